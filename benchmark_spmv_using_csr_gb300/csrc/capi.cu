@@ -92,6 +92,8 @@ struct bhsp_plan {
     bool one_head = false;  // the tile kernels take the one-head chunk form
     int x_sampled = 0, x_near = 0;  // sampled non-zeros, those with a near column
     bool x_l2 = false;              // the tile kernels gather x from L2 only
+    RowForm rows{};                 // lanes > 0: the row kernel runs, unless ...
+    bool variant_set = false;       // ... the caller forced a tile-kernel variant or grid
     int device = 0;
     std::string last_error;
 };
@@ -178,28 +180,51 @@ static int plan_build(bhsp_plan* p, cudaStream_t st) {
     //  - the x gather path: the locality of the columns on about 2^20 sampled non-zeros.
     const int cw = p->cfg.seg == 8 ? 4 : 8;
     const int step = p->nnz > (1 << 20) ? p->nnz / (1 << 20) : 1;
-    uint32_t* counts = nullptr;
-    uint32_t h[3] = {0u, 0u, 0u};
-    PLAN_CUDA(p, cudaMalloc(&counts, 3 * sizeof(uint32_t)));
-    cudaError_t e = launch_short_rows(p->row_ptr, p->m, cw, counts, st);
+    struct Counts {
+        RowCounts rows;
+        uint32_t locality[2];
+    } h = {};
+    Counts* counts = nullptr;
+    PLAN_CUDA(p, cudaMalloc(&counts, sizeof h));
+    cudaError_t e = launch_row_counts(p->row_ptr, p->m, cw, &counts->rows, st);
     if (e == cudaSuccess)
-        e = launch_x_locality(p->row_ptr, p->col, p->m, p->nnz, step, counts + 1, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(h, counts, sizeof h, cudaMemcpyDeviceToHost, st);
+        e = launch_x_locality(p->row_ptr, p->col, p->m, p->nnz, step, counts->locality, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, counts, sizeof h, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     cudaFree(counts);
     if (e != cudaSuccess) return cuda_fail(&p->last_error, e, "plan counts");
-    p->short_rows = (int)h[0];
-    p->one_head = one_head_pays(h[0], p->nnz, cw);
-    p->x_sampled = (int)h[1];
-    p->x_near = (int)h[2];
-    p->x_l2 = x_l2_pays(h[1], h[2]);
+    p->short_rows = (int)h.rows.short_rows;
+    p->one_head = one_head_pays(p->short_rows, p->nnz, cw);
+    p->x_sampled = (int)h.locality[0];
+    p->x_near = (int)h.locality[1];
+    p->x_l2 = x_l2_pays(h.locality[0], h.locality[1]);
+    p->rows = choose_row_form(h.rows, p->m, p->nnz, p->x_l2, p->vt == BHSP_VALUE_F64);
     return BHSPARSE_SUCCESS;
+}
+
+// Whether an execute runs the row kernel (one launch, no carry records).
+static bool plan_takes_rows(const bhsp_plan* p) {
+    return p->rows.lanes > 0 && !p->variant_set && p->grid_mode < 0;
 }
 
 static int plan_execute(bhsp_plan* p, const void* val, const void* x, void* y, cudaStream_t st,
                         int phase = 3) {
     if (p->m == 0) return BHSPARSE_SUCCESS;
     cudaError_t e = cudaSuccess;
+    if (plan_takes_rows(p)) {
+        if (phase & 1) {
+            const RowLaunch l{p->row_ptr, p->col,    val,  x,      y,      p->ticket,
+                              p->err,     p->m, p->nnz, p->rows};
+            switch (p->vt) {
+                case BHSP_VALUE_F64: e = launch_rows_f64(l, st); break;
+                case BHSP_VALUE_F32: e = launch_rows_f32(l, st); break;
+                case BHSP_VALUE_MIXED_F32: e = launch_rows_mixed_f32(l, st); break;
+                default: e = launch_rows_mixed_bf16(l, st); break;
+            }
+        }
+        if (e != cudaSuccess) return cuda_fail(&p->last_error, e, "SpMV launch");
+        return BHSPARSE_SUCCESS;
+    }
     switch (p->vt) {
         case BHSP_VALUE_F64:
         case BHSP_VALUE_F32: {
@@ -344,7 +369,7 @@ extern "C" int bhsp_plan_check(bhsp_plan* p, void* stream) {
 
 extern "C" int bhsp_plan_launches(const bhsp_plan* p) {
     if (!p) return 0;
-    return p->m == 0 ? 0 : (p->nworkers > 0 ? 2 : 1);
+    return p->m == 0 ? 0 : (p->nworkers > 0 && !plan_takes_rows(p) ? 2 : 1);
 }
 
 extern "C" int bhsp_plan_tiles(const bhsp_plan* p, const uint32_t** d_tile_ptr, int* ntiles,
@@ -376,6 +401,7 @@ extern "C" int bhsp_plan_set_variant(bhsp_plan* p, int one_head, int l2_only) {
         return BHSPARSE_INVALID_ARGUMENT;
     if (one_head >= 0) p->one_head = one_head == 1;
     if (l2_only >= 0) p->x_l2 = l2_only == 1;
+    if (one_head >= 0 || l2_only >= 0) p->variant_set = true;
     return BHSPARSE_SUCCESS;
 }
 

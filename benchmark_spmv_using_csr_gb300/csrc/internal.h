@@ -37,8 +37,16 @@ cudaError_t launch_partition(const int* row_ptr, int m, int nnz, int tile, uint3
                              cudaStream_t st);
 cudaError_t launch_bitflags(const int* row_ptr, int m, int nnz, int seg, const uint32_t* tile_ptr,
                             uint32_t* words, cudaStream_t st);
-// *count = non-empty rows shorter than cw non-zeros (zeroed first)
-cudaError_t launch_short_rows(const int* row_ptr, int m, int cw, uint32_t* count, cudaStream_t st);
+// What the plans' kernel choices need of the row lengths (one pass over row_ptr).
+struct RowCounts {
+    unsigned long long short_rows;  // non-empty rows shorter than cw non-zeros
+    unsigned long long max_len;     // the longest row
+    unsigned long long eights;      // non-empty rows of a multiple of 8 non-zeros
+    // over the passes of 32 / T consecutive rows, T = 1, 2, 4, 8: the sum of ceil(longest / 4T),
+    // the groups of 4 slots that the row kernel's lanes walk with T lanes to a row
+    unsigned long long groups[4];
+};
+cudaError_t launch_row_counts(const int* row_ptr, int m, int cw, RowCounts* counts, cudaStream_t st);
 // counts[0] = sampled non-zeros (every step-th), counts[1] = those whose column lies within 4 of
 // the previous entry of its row or of the entry at the same position of the previous row
 // (zeroed first)
@@ -55,6 +63,30 @@ inline bool one_head_pays(long long short_rows, long long nnz, int cw) {
     const long long chunks = (nnz + 32LL * cw - 1) / (32LL * cw);
     return 4 * short_rows <= chunks;
 }
+// The row kernel's lane layout for a matrix (lanes == 0: the matrix takes the tile kernels).
+struct RowForm {
+    int lanes = 0;        // lanes per row
+    int groups = 0;       // groups of 4 non-zeros per lane
+    bool rotate = false;  // rows start in the same shared-memory banks: spread their first slots
+};
+RowForm choose_row_form(const RowCounts& c, int m, int nnz, bool x_l2, bool f64);  // partition.cu
+// rows_<value type>.cu
+struct RowLaunch {
+    const int* row_ptr;
+    const int* col;
+    const void* val;
+    const void* x;
+    void* y;
+    int* ticket;
+    uint32_t* err;
+    int m, nnz;
+    RowForm form;
+};
+cudaError_t launch_rows_f64(const RowLaunch& l, cudaStream_t st);
+cudaError_t launch_rows_f32(const RowLaunch& l, cudaStream_t st);
+cudaError_t launch_rows_mixed_f32(const RowLaunch& l, cudaStream_t st);
+cudaError_t launch_rows_mixed_bf16(const RowLaunch& l, cudaStream_t st);
+
 cudaError_t launch_validate(const int* row_ptr, const int* col, int m, int n, int nnz,
                             uint32_t* bad, cudaStream_t st);
 

@@ -123,20 +123,47 @@ cudaError_t launch_bitflags(const int* row_ptr, int m, int nnz, int seg, const u
     return cudaGetLastError();
 }
 
-// Non-empty rows shorter than cw non-zeros.  Only such a row puts two row heads into one
-// lane's chunk of cw slots (heads at s and s + len share an aligned chunk only if len < cw), and
-// it does so in at most one chunk.
-__global__ void k_short_rows(const int* __restrict__ row_ptr, int m, int cw,
-                             uint32_t* __restrict__ count) {
+// One thread per row (a warp: 32 consecutive rows, aligned).
+//  * Non-empty rows shorter than cw non-zeros.  Only such a row puts two row heads into one lane's
+//    chunk of cw slots (heads at s and s + len share an aligned chunk only if len < cw), and it
+//    does so in at most one chunk.
+//  * What the row kernel needs: see RowCounts.
+__global__ void k_row_counts(const int* __restrict__ row_ptr, int m, int cw,
+                             RowCounts* __restrict__ counts) {
     const long long stride = (long long)gridDim.x * blockDim.x;  // 64-bit: m may be near 2^31
-    uint32_t c = 0;
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < m; r += stride) {
-        const int len = __ldg(row_ptr + r + 1) - __ldg(row_ptr + r);
-        c += (len > 0 && len < cw) ? 1u : 0u;
+    const int lane = threadIdx.x & 31;
+    unsigned shorts = 0, top = 0, eights = 0;
+    unsigned long long groups[4] = {0, 0, 0, 0};
+    for (long long r0 = blockIdx.x * (long long)blockDim.x + threadIdx.x - lane; r0 < m;
+         r0 += stride) {  // warp-uniform
+        const long long r = r0 + lane;
+        const int len = r < m ? __ldg(row_ptr + r + 1) - __ldg(row_ptr + r) : 0;
+        shorts += (len > 0 && len < cw) ? 1u : 0u;
+        eights += (len > 0 && len % 8 == 0) ? 1u : 0u;
+        int most = len;  // the longest row of 4, 8, 16 and then 32 consecutive ones
+#pragma unroll
+        for (int t = 3, d = 1; t >= 0; --t) {
+            const int rows = 32 >> t;
+            for (; d < rows; d <<= 1) most = max(most, __shfl_xor_sync(SPMV_FULL_MASK, most, d));
+            if ((lane & (rows - 1)) == 0) groups[t] += (unsigned)((most + (4LL << t) - 1) >> (2 + t));
+        }
+        top = max(top, (unsigned)most);
     }
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) c += __shfl_xor_sync(SPMV_FULL_MASK, c, d);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
+    for (int d = 16; d > 0; d >>= 1) {
+        shorts += __shfl_xor_sync(SPMV_FULL_MASK, shorts, d);
+        eights += __shfl_xor_sync(SPMV_FULL_MASK, eights, d);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) groups[t] += __shfl_xor_sync(SPMV_FULL_MASK, groups[t], d);
+    }
+    if (lane == 0) {
+        if (shorts) atomicAdd(&counts->short_rows, (unsigned long long)shorts);
+        if (eights) atomicAdd(&counts->eights, (unsigned long long)eights);
+        if (top) atomicMax(&counts->max_len, (unsigned long long)top);
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+            if (groups[t]) atomicAdd(&counts->groups[t], groups[t]);
+    }
 }
 
 // Locality of the columns for the x gathers, on every step-th non-zero: near when its column is
@@ -193,11 +220,37 @@ cudaError_t launch_x_locality(const int* row_ptr, const int* col, int m, int nnz
     return cudaGetLastError();
 }
 
-cudaError_t launch_short_rows(const int* row_ptr, int m, int cw, uint32_t* count, cudaStream_t st) {
-    cudaError_t e = cudaMemsetAsync(count, 0, sizeof(uint32_t), st);
+cudaError_t launch_row_counts(const int* row_ptr, int m, int cw, RowCounts* counts,
+                              cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(counts, 0, sizeof(RowCounts), st);
     if (e != cudaSuccess) return e;
-    if (m > 0) k_short_rows<<<grid_for(m, 256, 8), 256, 0, st>>>(row_ptr, m, cw, count);
+    if (m > 0) k_row_counts<<<grid_for(m, 256, 8), 256, 0, st>>>(row_ptr, m, cw, counts);
     return cudaGetLastError();
+}
+
+// Whether a matrix takes the row kernel, and with which lane layout.
+//  * Columns with locality (x_l2 false): lanes on rows pay through coalesced x reads, which random
+//    columns do not have (a power-law or uniform-density matrix ran 1.2-4x slower here).
+//  * The longest row fits in T = 8 lanes of 28 slots (224 non-zeros), FP64 in 32 non-zeros: its
+//    slots beyond the row's end cost as much of the narrow FP64 pipe as real ones, and with 2 or
+//    more lanes to a row it was 0.86-1.1x the tile kernel.
+//  * The rows fill the slots that their pass walks.  Measured against the tile kernel at the best
+//    of six schedules on banded matrices of 1e6-4e7 non-zeros (time tile / time rows): from a
+//    share of 0.6 on 0.97-1.8x in FP32, 0.97-1.7x in mixed FP32, 1.1-2.0x in BF16 storage (0.5
+//    and below: 0.87-1.2x); in FP64 with rows of up to 12 non-zeros 1.1-1.9x, with longer ones
+//    1.0-1.5x from 0.84 on and 0.73-0.98x below.
+RowForm choose_row_form(const RowCounts& c, int m, int nnz, bool x_l2, bool f64) {
+    RowForm f;
+    // the kernel counts rows in whole passes of 32: their numbers must not pass 2^31
+    if (x_l2 || nnz == 0 || m > 0x7fffff00 || c.max_len > (f64 ? 32u : 224u)) return f;
+    int t = 0;  // log2 of the lanes per row
+    while (c.max_len > (28ull << t)) ++t;
+    const double slots = 128.0 * (double)c.groups[t];
+    if ((double)nnz < (f64 && c.max_len > 12 ? 0.84 : 0.6) * slots) return f;
+    f.lanes = 1 << t;
+    f.groups = (int)((c.max_len + (4u << t) - 1) >> (2 + t));
+    f.rotate = 2 * c.eights > (unsigned long long)m;
+    return f;
 }
 
 cudaError_t launch_validate(const int* row_ptr, const int* col, int m, int n, int nnz,

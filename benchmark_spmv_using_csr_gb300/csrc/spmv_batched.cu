@@ -416,20 +416,24 @@ extern "C" int bhsp_batch_create(bhsp_batch** out, int count, int m_total, int n
         // width of the batched kernel, and the locality of about 2^20 sampled columns
         const int cw = k == 8 ? 2 : (c.seg == 8 || k == 4) ? 4 : 8;  // chunk_width<S, x entry>
         const int step = nnz_total > (1 << 20) ? nnz_total / (1 << 20) : 1;
-        uint32_t* counts = nullptr;
-        uint32_t h[3] = {0u, 0u, 0u};
-        e = cudaMalloc(&counts, 3 * sizeof(uint32_t));
-        if (e == cudaSuccess) e = launch_short_rows(d_row_ptr, m_total, cw, counts, st);
+        struct Counts {
+            RowCounts rows;
+            uint32_t locality[2];
+        } h = {};
+        Counts* counts = nullptr;
+        e = cudaMalloc(&counts, sizeof h);
+        if (e == cudaSuccess) e = launch_row_counts(d_row_ptr, m_total, cw, &counts->rows, st);
         if (e == cudaSuccess)
-            e = launch_x_locality(d_row_ptr, d_col_idx, m_total, nnz_total, step, counts + 1, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(h, counts, sizeof h, cudaMemcpyDeviceToHost, st);
+            e = launch_x_locality(d_row_ptr, d_col_idx, m_total, nnz_total, step, counts->locality,
+                                  st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&h, counts, sizeof h, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         cudaFree(counts);
-        b->short_rows = (int)h[0];
-        b->x_sampled = (int)h[1];
-        b->x_near = (int)h[2];
-        b->var.one_head = k == 1 && one_head_pays(h[0], nnz_total, cw);
-        b->var.x_l2 = x_l2_pays(h[1], h[2]);
+        b->short_rows = (int)h.rows.short_rows;
+        b->x_sampled = (int)h.locality[0];
+        b->x_near = (int)h.locality[1];
+        b->var.one_head = k == 1 && one_head_pays(b->short_rows, nnz_total, cw);
+        b->var.x_l2 = x_l2_pays(h.locality[0], h.locality[1]);
     }
     b->grid = e == cudaSuccess ? batch_grid(k, c, b->var) : 0;
     const size_t nw = b->nworkers > 0 ? (size_t)b->nworkers : 1;

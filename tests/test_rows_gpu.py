@@ -1,0 +1,128 @@
+"""The row kernel (lanes assigned to whole rows), which a plan takes for matrices whose rows are
+short, of much the same length and with columns of some locality: bit for bit against an int64
+sum on integer-valued data, at the edges of its lane layouts (1 to 8 lanes per row, 1 to 7 groups
+of 4 slots each), of its passes of 32 lanes and of the bulk copies' groups of 8 non-zeros."""
+import numpy as np
+import pytest
+
+import benchmark_spmv_using_csr_gb300 as sp
+
+pytestmark = pytest.mark.gpu
+
+VTS = [sp.VALUE_F64, sp.VALUE_F32, sp.VALUE_MIXED_F32, sp.VALUE_MIXED_BF16]
+# longest row: 1 lane up to 28, 2 up to 56, 4 up to 112, 8 up to 224; FP64 up to 32
+LENGTHS = [1, 4, 5, 8, 9, 12, 13, 16, 17, 20, 24, 25, 28, 29, 32, 33, 48, 56, 57, 64, 112, 113, 224]
+
+
+def banded(torch, lens, seed):
+    """Rows of the given lengths whose columns run on from the row's number (modulo m)."""
+    m = lens.size
+    rp = np.zeros(m + 1, np.int32)
+    rp[1:] = np.cumsum(lens)
+    row = np.repeat(np.arange(m), lens)
+    col = ((row + np.arange(row.size) - rp[row]) % m).astype(np.int32)
+    rng = np.random.default_rng(seed)
+    val = rng.integers(-4, 5, row.size).astype(np.float64)
+    x = rng.integers(-4, 5, m).astype(np.float64)
+    y = np.zeros(m)
+    np.add.at(y, row, val * x[col])
+    return rp, col, val, x, y
+
+
+def device(torch, vt, a):
+    store = {sp.VALUE_F64: torch.float64, sp.VALUE_MIXED_BF16: torch.bfloat16}.get(vt, torch.float32)
+    vec = torch.float64 if vt == sp.VALUE_F64 else torch.float32
+    rp, col, val, x, _ = a
+    return (torch.from_numpy(rp).cuda(), torch.from_numpy(col).cuda(),
+            torch.from_numpy(val).cuda().to(store), torch.from_numpy(x).cuda().to(vec),
+            torch.full((x.size,), float("nan"), dtype=vec, device="cuda"))
+
+
+@pytest.mark.parametrize("vt", VTS)
+@pytest.mark.parametrize("m", [1, 3, 31, 32, 33, 1001])
+def test_lane_layouts_bit_exact(cuda_ok, vt, m):
+    """Every layout, with all rows at the longest length and with some shorter and empty ones (at
+    the start, the end and between), twice: y must not depend on what it held."""
+    import torch
+    for top in LENGTHS:
+        whole = np.full(m, top)
+        mixed = whole.copy()
+        mixed[m // 2::7] -= min(2, top - 1)
+        mixed[3::50] = 0
+        if m > 1000:
+            mixed[:2] = mixed[-40:] = 0
+        for lens in (whole, mixed):
+            a = banded(torch, lens, 10 * top + m)
+            rp, col, val, x, y = device(torch, vt, a)
+            p = sp.Plan(vt, m, m, rp, col)
+            if vt != sp.VALUE_F64 and m > 1000 and top not in (1, 5, 9, 13):
+                assert p.launches == 1, (top, "the row kernel")
+            for _ in range(2):
+                p.execute(val, x, y)
+                p.check()
+                bad = int((y.cpu().double().numpy() != a[4]).sum())
+                assert bad == 0, (top, bad)
+                y.fill_(float("nan"))
+            p.close()
+
+
+@pytest.mark.parametrize("vt", VTS)
+def test_many_passes_per_warp_bit_exact(cuda_ok, vt):
+    """More passes than warps: the strided workers, and for FP64 the ticket, whose last warp leaves
+    it at zero for the next launch.  A forced variant or grid sends the same plan to the tile
+    kernel, with the same y."""
+    import torch
+    m = 900_001
+    lens = np.full(m, 27)
+    lens[::160] = lens[159::160] = 18
+    a = banded(torch, lens, 5)
+    rp, col, val, x, y = device(torch, vt, a)
+    p = sp.Plan(vt, m, m, rp, col)
+    assert p.launches == 1
+    want = torch.from_numpy(a[4]).cuda().to(y.dtype)
+    for _ in range(3):
+        y.fill_(float("nan"))
+        p.execute(val, x, y)
+        p.check()
+        assert torch.equal(y, want)
+    p.set_grid(False)
+    assert p.launches == 2
+    y.fill_(float("nan"))
+    p.execute(val, x, y)
+    p.check()
+    assert torch.equal(y, want)
+    p.set_grid(None)
+    assert p.launches == 1
+    p.set_variant(l2_only=False)
+    assert p.launches == 2
+    p.close()
+
+
+def test_row_kernel_decision(cuda_ok):
+    """Short rows of one length with near columns take the row kernel; random columns, one long
+    row, and rows that would leave most slots empty do not."""
+    import torch
+    rng = np.random.default_rng(1)
+
+    def launches(lens, vt=sp.VALUE_F32, spread=False):
+        rp, col = banded(torch, lens, 2)[:2]
+        if spread:
+            col = rng.integers(0, lens.size, col.size).astype(np.int32)
+        p = sp.Plan(vt, lens.size, lens.size, torch.from_numpy(rp).cuda(), torch.from_numpy(col).cuda())
+        try:
+            return p.launches
+        finally:
+            p.close()
+
+    m = 20_000
+    whole = np.full(m, 27)
+    assert launches(whole) == 1 and launches(whole, sp.VALUE_F64) == 1
+    assert launches(whole, spread=True) == 2
+    one_long = whole.copy()
+    one_long[77] = 225
+    assert launches(one_long) == 2
+    assert launches(np.full(m, 33), sp.VALUE_F64) == 2 and launches(np.full(m, 33)) == 1
+    uneven = rng.integers(0, 28, m)
+    assert launches(uneven) == 2
+    three_quarters = rng.integers(20, 28, m)  # 24 of 28 slots on average
+    assert launches(three_quarters) == 1
