@@ -139,6 +139,58 @@ cudaError_t launch_convert_from_f64(const double* src, void* dst, size_t n, bool
                                     cudaStream_t st);
 cudaError_t launch_convert_to_f64(const float* src, double* dst, size_t n, cudaStream_t st);
 
+// The batched form: its buffers, and the work lists of its two kernels (batch_kernel.cuh).
+struct BatchLaunch {
+    const int* row_ptr;
+    const int* col;
+    const float* val;
+    const void* x;
+    void* y;
+    const uint32_t* tile_ptr;
+    int* rec_row;
+    void* rec_val;
+    uint32_t* err;
+    int* ticket;
+    int m, n, nnz;
+};
+// A row worker: rows [first, last) with 1 << (form & 7) lanes per row (bit 3: rotated slots); or,
+// form < 0, the carry records [first, last) of the tile workers to add to their rows.
+struct RowWork {
+    int form, first, last;
+};
+// A tile worker: tiles [first, last) of the run of rows [row0, row1), its part of tile_ptr (tile t's
+// entry is tile_ptr[at + t]); its carry record has the worker's number.
+struct TileWork {
+    int first, last, row0, row1, at;
+};
+constexpr int BATCH_SLOTS = 28;  // of a lane in a pass: rows of up to 28, 56, 112, 224 non-zeros
+// The two work lists and their kernels' buffers.
+struct BatchWork {
+    TileWork* tiles = nullptr;  // [ntiles]
+    RowWork* rows = nullptr;    // [nrows], the carry records' workers last
+    uint32_t* tile_ptr = nullptr;
+    int* rec_row = nullptr;     // [ntiles]
+    void* rec_val = nullptr;
+    int* row_ticket = nullptr;  // [2], as the tile kernel's
+    int ntiles = 0, nrows = 0, tiles_grid = 0, rows_grid = 0;
+};
+// What the work lists need of each block of 256 rows.
+struct BlockStat {
+    int first;      // its first non-zero
+    int max_len;    // the longest row
+    int groups[4];  // as RowCounts::groups, over this block
+    int eights;     // non-empty rows of a multiple of 8 non-zeros
+    int filled;     // non-empty rows
+};
+constexpr int BATCH_BLOCK = 256;
+cudaError_t launch_block_stats(const int* row_ptr, int m, BlockStat* stat, cudaStream_t st);
+// A run of rows for the tile workers: tiles [t0, t1], boundary t at tile_ptr[at + t - t0].
+struct TileRun {
+    int row0, row1, t0, t1, at;
+};
+cudaError_t launch_run_tiles(const int* row_ptr, const TileRun* runs, int nruns, int nbounds,
+                             int tile, uint32_t* tile_ptr, cudaStream_t st);
+
 inline bool is_supported_value_type(int vt) { return vt >= 0 && vt <= 3; }
 
 }  // namespace spmv

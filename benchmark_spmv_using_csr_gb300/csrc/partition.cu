@@ -228,6 +228,77 @@ cudaError_t launch_row_counts(const int* row_ptr, int m, int cw, RowCounts* coun
     return cudaGetLastError();
 }
 
+// One warp per block of 256 rows.
+__global__ void k_block_stats(const int* __restrict__ row_ptr, int m, int nblocks,
+                              BlockStat* __restrict__ stat) {
+    const int lane = threadIdx.x & 31;
+    const int nwarps = gridDim.x * (blockDim.x >> 5);
+    for (int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); b < nblocks; b += nwarps) {
+        BlockStat s{};
+        s.first = __ldg(row_ptr + b * BATCH_BLOCK);
+        for (int i = 0; i < BATCH_BLOCK; i += 32) {
+            const long long r = (long long)b * BATCH_BLOCK + i + lane;
+            const int lo = r < m ? __ldg(row_ptr + r) : 0;
+            const int len = r < m ? __ldg(row_ptr + r + 1) - lo : 0;
+            s.filled += __popc(__ballot_sync(SPMV_FULL_MASK, len > 0));
+            s.eights += __popc(__ballot_sync(SPMV_FULL_MASK, len > 0 && len % 8 == 0));
+            int most = len;
+#pragma unroll
+            for (int t = 3, d = 1; t >= 0; --t) {
+                const int rows = 32 >> t;
+                for (; d < rows; d <<= 1) most = max(most, __shfl_xor_sync(SPMV_FULL_MASK, most, d));
+                s.groups[t] += (lane & (rows - 1)) == 0 ? (int)((most + (4LL << t) - 1) >> (2 + t)) : 0;
+            }
+            s.max_len = max(s.max_len, most);
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) s.groups[t] = __reduce_add_sync(SPMV_FULL_MASK, s.groups[t]);
+        if (lane == 0) stat[b] = s;
+    }
+}
+
+// One thread per tile boundary of every run (as k_tile_rows, on the run's rows; the first
+// boundary is the run's first row, so that its leading empty rows lie in a span).
+__global__ void k_run_tiles(const int* __restrict__ row_ptr, const TileRun* __restrict__ runs,
+                            int nruns, int nbounds, int tile, uint32_t* __restrict__ tile_ptr) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nbounds) return;
+    int lo = 0, hi = nruns - 1;  // the run of boundary i: the last one with at <= i
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (runs[mid].at <= i)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    const TileRun r = runs[lo];
+    const int t = r.t0 + i - r.at;
+    const int m = r.row1 - r.row0;
+    if (t == r.t0) {
+        tile_ptr[i] = 0u;
+        return;
+    }
+    const int end = __ldg(row_ptr + r.row1);
+    const long long key = min((long long)t * tile, (long long)end);
+    tile_ptr[i] = (uint32_t)(search_right(row_ptr + r.row0, (int)key, m + 1) - 1);
+}
+
+cudaError_t launch_block_stats(const int* row_ptr, int m, BlockStat* stat, cudaStream_t st) {
+    const int nblocks = (int)(((long long)m + BATCH_BLOCK - 1) / BATCH_BLOCK);
+    if (nblocks > 0)
+        k_block_stats<<<grid_for((long long)nblocks * 32, 256, 8), 256, 0, st>>>(row_ptr, m,
+                                                                                nblocks, stat);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_run_tiles(const int* row_ptr, const TileRun* runs, int nruns, int nbounds,
+                             int tile, uint32_t* tile_ptr, cudaStream_t st) {
+    if (nbounds > 0)
+        k_run_tiles<<<(nbounds + 255) / 256, 256, 0, st>>>(row_ptr, runs, nruns, nbounds, tile,
+                                                           tile_ptr);
+    return cudaGetLastError();
+}
+
 // Whether a matrix takes the row kernel, and with which lane layout.
 //  * Columns with locality (x_l2 false): lanes on rows pay through coalesced x reads, which random
 //    columns do not have (a power-law or uniform-density matrix ran 1.2-4x slower here).

@@ -18,185 +18,9 @@
 
 #include "../../include/spmv_gb300.h"
 #include "internal.h"
-#include "tile_kernel.cuh"
+#include "policies_batched.cuh"
 
 namespace spmv {
-
-// ---- k interleaved FP32 values, accumulators and FP64 records ----
-template <int K>
-struct alignas(4 * K) VecF {
-    float v[K];
-    __device__ VecF() {}
-    __device__ explicit VecF(int z) {
-#pragma unroll
-        for (int j = 0; j < K; ++j) v[j] = (float)z;
-    }
-};
-template <int K>
-struct VecD {
-    double v[K];
-};
-template <int K>
-struct AccK {
-    float2 v[K];
-};
-
-__device__ __forceinline__ VecF<1> ld_x(const VecF<1>* p, uint64_t) {
-    VecF<1> r;
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(r.v[0]) : "l"(p));
-    return r;
-}
-__device__ __forceinline__ VecF<2> ld_x(const VecF<2>* p, uint64_t) {
-    VecF<2> r;
-    asm volatile("ld.global.nc.v2.f32 {%0,%1}, [%2];" : "=f"(r.v[0]), "=f"(r.v[1]) : "l"(p));
-    return r;
-}
-__device__ __forceinline__ VecF<4> ld_x(const VecF<4>* p, uint64_t) {
-    VecF<4> r;
-    asm volatile("ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%4];"
-                 : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3])
-                 : "l"(p));
-    return r;
-}
-__device__ __forceinline__ VecF<8> ld_x(const VecF<8>* p, uint64_t) {
-    VecF<8> r;
-    asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]), "=f"(r.v[4]),
-                   "=f"(r.v[5]), "=f"(r.v[6]), "=f"(r.v[7])
-                 : "l"(p));
-    return r;
-}
-
-// the same gathers from L2 only (ld.global.cg), the batch's plan choice when its columns have no
-// locality
-__device__ __forceinline__ VecF<1> ld_x_l2(const VecF<1>* p) {
-    VecF<1> r;
-    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(r.v[0]) : "l"(p));
-    return r;
-}
-__device__ __forceinline__ VecF<2> ld_x_l2(const VecF<2>* p) {
-    VecF<2> r;
-    asm volatile("ld.global.cg.v2.f32 {%0,%1}, [%2];" : "=f"(r.v[0]), "=f"(r.v[1]) : "l"(p));
-    return r;
-}
-__device__ __forceinline__ VecF<4> ld_x_l2(const VecF<4>* p) {
-    VecF<4> r;
-    asm volatile("ld.global.cg.v4.f32 {%0,%1,%2,%3}, [%4];"
-                 : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3])
-                 : "l"(p));
-    return r;
-}
-__device__ __forceinline__ VecF<8> ld_x_l2(const VecF<8>* p) {
-    VecF<8> r;
-    asm volatile("ld.global.cg.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]), "=f"(r.v[4]),
-                   "=f"(r.v[5]), "=f"(r.v[6]), "=f"(r.v[7])
-                 : "l"(p));
-    return r;
-}
-
-template <int K>
-__device__ __forceinline__ AccK<K> sh_down(const AccK<K>& a, int d) {
-    AccK<K> r;
-#pragma unroll
-    for (int j = 0; j < K; ++j) r.v[j] = sh_down(a.v[j], d);
-    return r;
-}
-template <int K>
-__device__ __forceinline__ AccK<K> sh_idx(const AccK<K>& a, int s) {
-    AccK<K> r;
-#pragma unroll
-    for (int j = 0; j < K; ++j) r.v[j] = sh_idx(a.v[j], s);
-    return r;
-}
-template <int K>
-__device__ __forceinline__ AccK<K> sh_xor(const AccK<K>& a, int d) {
-    AccK<K> r;
-#pragma unroll
-    for (int j = 0; j < K; ++j) r.v[j] = sh_xor(a.v[j], d);
-    return r;
-}
-
-// compensated float-float steps (TwoProduct by FMA + Knuth TwoSum), rounded explicitly
-__device__ __forceinline__ float2 ffk_add_product(float v, float x, float2 a) {
-    const float p = __fmul_rn(v, x);
-    const float ep = __fmaf_rn(v, x, -p);
-    const float s = __fadd_rn(a.x, p);
-    const float bb = __fsub_rn(s, a.x);
-    const float es = __fadd_rn(__fsub_rn(a.x, __fsub_rn(s, bb)), __fsub_rn(p, bb));
-    return make_float2(s, __fadd_rn(a.y, __fadd_rn(es, ep)));
-}
-__device__ __forceinline__ float2 ffk_add(float2 a, float2 b) {
-    const float s = __fadd_rn(a.x, b.x);
-    const float bb = __fsub_rn(s, a.x);
-    const float es = __fadd_rn(__fsub_rn(a.x, __fsub_rn(s, bb)), __fsub_rn(b.x, bb));
-    return make_float2(s, __fadd_rn(__fadd_rn(a.y, b.y), es));
-}
-
-// The mixed-FP32 arithmetic of spmv_mixed.cu applied to k right-hand sides at once.
-template <int K>
-struct PolMixedK {
-    using VS = float;
-    using VC = float;
-    using XT = VecF<K>;
-    using YT = VecF<K>;
-    using Acc = AccK<K>;
-    using Carry = AccK<K>;
-    using Rec = VecD<K>;
-    __device__ static Acc zero() {
-        Acc r;
-#pragma unroll
-        for (int j = 0; j < K; ++j) r.v[j] = make_float2(0.f, 0.f);
-        return r;
-    }
-    __device__ static Carry carry_zero() { return zero(); }
-    __device__ static Acc fma(float v, const XT& x, const Acc& a) {
-        Acc r;
-#pragma unroll
-        for (int j = 0; j < K; ++j) r.v[j] = ffk_add_product(v, x.v[j], a.v[j]);
-        return r;
-    }
-    __device__ static Acc add(const Acc& a, const Acc& b) {
-        Acc r;
-#pragma unroll
-        for (int j = 0; j < K; ++j) r.v[j] = ffk_add(a.v[j], b.v[j]);
-        return r;
-    }
-    __device__ static Carry carry_from(const Acc& a) { return a; }
-    __device__ static Acc carry_to_acc(const Carry& c) { return c; }
-    __device__ static Carry carry_add(const Carry& c, const Acc& a) { return add(c, a); }
-    __device__ static YT out_acc(const Acc& a) {
-        YT r;
-#pragma unroll
-        for (int j = 0; j < K; ++j) r.v[j] = __fadd_rn(a.v[j].x, a.v[j].y);
-        return r;
-    }
-    __device__ static YT out_carry(const Carry& c) { return out_acc(c); }
-    __device__ static Rec rec_from(const Carry& c) {
-        Rec r;
-#pragma unroll
-        for (int j = 0; j < K; ++j) r.v[j] = (double)c.v[j].x + (double)c.v[j].y;
-        return r;
-    }
-    __device__ static Rec rec_add(const Rec& a, const Rec& b) {
-        Rec r;
-#pragma unroll
-        for (int j = 0; j < K; ++j) r.v[j] = a.v[j] + b.v[j];
-        return r;
-    }
-    __device__ static Rec rec_of_y(const YT& y) {
-        Rec r;
-#pragma unroll
-        for (int j = 0; j < K; ++j) r.v[j] = (double)y.v[j];
-        return r;
-    }
-    __device__ static YT out_rec(const Rec& r) {
-        YT y;
-#pragma unroll
-        for (int j = 0; j < K; ++j) y.v[j] = __double2float_rn(r.v[j]);
-        return y;
-    }
-};
 
 // the persistent kernel for K right-hand sides: register-capped from 4 on.  OH (the one-head
 // chunk form) exists for one right-hand side only, whose accumulator is scalar.
@@ -229,20 +53,6 @@ static int persistent_grid() {
     return device_sm_count() * (per_sm > 0 ? per_sm : 1);
 }
 
-struct BatchLaunch {
-    const int* row_ptr;
-    const int* col;
-    const float* val;
-    const void* x;
-    void* y;
-    const uint32_t* tile_ptr;
-    int* rec_row;
-    void* rec_val;
-    uint32_t* err;
-    int* ticket;
-    int m, n, nnz;
-};
-
 // The plan's kernel variant: the one-head chunk form (one right-hand side, few short rows) and
 // L2-only x gathers (columns without locality), both chosen from counts made on the device.
 struct BatchVariant {
@@ -252,21 +62,7 @@ struct BatchVariant {
 
 template <int K, int S, int WARPS, bool OH, bool XL2>
 static cudaError_t enqueue_k(const BatchLaunch& l, int tpw, int grid, cudaStream_t st) {
-    TileArgs<PolMixedK<K>> a;
-    a.row_ptr = l.row_ptr;
-    a.col = l.col;
-    a.val = l.val;
-    a.x = static_cast<const VecF<K>*>(l.x);
-    a.y = static_cast<VecF<K>*>(l.y);
-    a.tile_ptr = l.tile_ptr;
-    a.rec_row = l.rec_row;
-    a.rec_val = static_cast<VecD<K>*>(l.rec_val);
-    a.err = l.err;
-    a.m = l.m;
-    a.n = l.n;
-    a.nnz = l.nnz;
-    a.phase = 3;
-    a.ticket = l.ticket;
+    const TileArgs<PolMixedK<K>> a = batch_tile_args<K>(l);
     const int nt = num_tiles(l.nnz, 32 * S);
     const int nw = (nt + tpw - 1) / tpw;
     return enqueue_batched<K, S, WARPS, OH, XL2>(a, tpw, nw, nt, grid, st);
@@ -351,6 +147,9 @@ struct bhsp_batch {
     void* rec_val = nullptr;
     uint32_t* err = nullptr;
     int* ticket = nullptr;
+    // the work lists of row and tile workers, taken when `mixed` is set and no variant was forced
+    bool mixed = false, variant_set = false;
+    BatchWork work{};
     // the graph and the buffers it was captured with
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -368,6 +167,13 @@ static void batch_release(bhsp_batch* b) {
     cudaFree(b->rec_val);
     cudaFree(b->err);
     cudaFree(b->ticket);
+    cudaFree(b->work.tiles);
+    cudaFree(b->work.rows);
+    cudaFree(b->work.tile_ptr);
+    cudaFree(b->work.rec_row);
+    cudaFree(b->work.rec_val);
+    cudaFree(b->work.row_ticket);
+    b->work = BatchWork{};
     b->exec = nullptr;
     b->graph = nullptr;
 }
@@ -376,6 +182,125 @@ static int batch_cuda(bhsp_batch* b, cudaError_t e, const char* what) {
     b->last_error = std::string(what) + ": " + cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? BHSPARSE_OUT_OF_MEMORY : BHSPARSE_CUDA_ERROR;
 }
+
+// The batch's work lists (see batch_kernel.cuh), from two right-hand sides on: row workers for the
+// blocks of 256 rows that suit lanes on whole rows, tile workers for the runs between them.  Leaves
+// b->mixed false where the row workers would hold less than a quarter of the batch.
+//  * One right-hand side keeps the one tile kernel: on the 64-matrix mix the two kernels took 131
+//    against 137 us, on 128 matrices 238 against 232 us.
+//  * A block suits the row workers where its longest row fits (224 non-zeros) and its rows fill 0.4
+//    of the slots that their passes walk.  Random columns are no bar here: an x entry is 8 to 32
+//    bytes, its own sector or a good part of one, whichever lane reads it.  64 matrices of
+//    uniform density (Poisson rows of up to 20, random columns): 167 -> 128, 247 -> 158 and 280 ->
+//    216 us at 2, 4 and 8 right-hand sides; thresholds of 0.2 to 0.5 differ by 3 %.
+static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
+    const int nblocks = (int)(((long long)b->m + BATCH_BLOCK - 1) / BATCH_BLOCK);
+    // (row numbers of whole passes must not pass 2^31)
+    if (b->k == 1 || b->nnz == 0 || b->m > 0x7fffff00) return cudaSuccess;
+    std::vector<BlockStat> stat((size_t)nblocks);
+    BlockStat* d_stat = nullptr;
+    cudaError_t e = cudaMalloc(&d_stat, sizeof(BlockStat) * (size_t)nblocks);
+    if (e == cudaSuccess) e = launch_block_stats(b->row_ptr, b->m, d_stat, st);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(stat.data(), d_stat, sizeof(BlockStat) * (size_t)nblocks,
+                            cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    cudaFree(d_stat);
+    if (e != cudaSuccess) return e;
+    auto nnz_to = [&](int i) { return i < nblocks ? stat[(size_t)i].first : b->nnz; };
+    // the row form of a block, or -1
+    auto form_of = [&](int i) -> int {
+        const BlockStat& s = stat[(size_t)i];
+        const int nnz = nnz_to(i + 1) - s.first;
+        if (nnz == 0) return 0;
+        if (s.max_len > 8 * BATCH_SLOTS) return -1;
+        int t = 0;
+        while (s.max_len > BATCH_SLOTS << t) ++t;
+        if (nnz < 0.4 * 128.0 * s.groups[t]) return -1;
+        return t | (2 * s.eights > s.filled ? 8 : 0);
+    };
+    std::vector<int> form((size_t)nblocks);
+    long long row_nnz = 0;
+    for (int i = 0; i < nblocks; ++i) {
+        form[(size_t)i] = form_of(i);
+        if (form[(size_t)i] >= 0) row_nnz += nnz_to(i + 1) - stat[(size_t)i].first;
+    }
+    if (4 * row_nnz < b->nnz) return cudaSuccess;
+    const int tile = 32 * b->cfg.seg;
+    const long long warps = (long long)device_sm_count() * 16;
+    // passes per row worker (up to 2) and tiles per tile worker (up to 1024 non-zeros), as many as
+    // leave every warp several workers: on the 64-matrix mix 4 and 8 passes or 2048 and 4096
+    // non-zeros were 0-5 % slower, on 5 and 16 matrices up to 38 %
+    long long passes = 0;
+    for (int i = 0; i < nblocks; ++i)
+        if (form[(size_t)i] >= 0) passes += BATCH_BLOCK / 32 << (form[(size_t)i] & 7);
+    const int ppw = (int)std::min<long long>(std::max<long long>(passes / (6 * warps), 1), 2);
+    const int tpw = (int)std::min<long long>(
+        {b->cfg.tiles_per_worker, std::max(1024 / tile, 1),
+         (int)std::max<long long>((b->nnz - row_nnz) / tile / (6 * warps), 1)});
+    std::vector<RowWork> rows;
+    std::vector<TileWork> tiles;
+    std::vector<TileRun> runs;
+    int nbounds = 0;
+    for (int i = 0; i < nblocks;) {
+        const int f = form[(size_t)i];
+        int j = i + 1;
+        while (j < nblocks && form[(size_t)j] == f) ++j;
+        const int row0 = i * BATCH_BLOCK;
+        const int row1 = (int)std::min<long long>((long long)j * BATCH_BLOCK, b->m);
+        if (f >= 0) {
+            const int step = std::max(ppw * (32 >> (f & 7)), 1);
+            for (long long r = row0; r < row1; r += step)
+                rows.push_back(RowWork{f, (int)r, (int)std::min<long long>(r + step, row1)});
+        } else {
+            TileRun r{row0, row1, nnz_to(i) / tile, (int)(((long long)nnz_to(j) + tile - 1) / tile),
+                      nbounds};
+            nbounds += r.t1 - r.t0 + 1;
+            runs.push_back(r);
+            for (int t = r.t0; t < r.t1; t += tpw)
+                tiles.push_back(TileWork{t, std::min(t + tpw, r.t1), row0, row1, r.at - r.t0});
+        }
+        i = j;
+    }
+    for (int i = 0; i < (int)tiles.size(); i += 32)
+        rows.push_back(RowWork{-1, i, std::min(i + 32, (int)tiles.size())});
+    BatchWork& w = b->work;
+    w.ntiles = (int)tiles.size();
+    w.nrows = (int)rows.size();
+    TileRun* d_runs = nullptr;
+    e = cudaMalloc(&w.rows, sizeof(RowWork) * rows.size());
+    if (e == cudaSuccess) e = cudaMalloc(&w.tiles, sizeof(TileWork) * (tiles.size() + 1));
+    if (e == cudaSuccess) e = cudaMalloc(&w.tile_ptr, sizeof(uint32_t) * (size_t)(nbounds + 1));
+    if (e == cudaSuccess) e = cudaMalloc(&w.rec_row, sizeof(int) * (tiles.size() + 1));
+    if (e == cudaSuccess) e = cudaMalloc(&w.rec_val, sizeof(double) * b->k * (tiles.size() + 1));
+    if (e == cudaSuccess) e = cudaMalloc(&w.row_ticket, 2 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMalloc(&d_runs, sizeof(TileRun) * (runs.size() + 1));
+    if (e == cudaSuccess) e = cudaMemsetAsync(w.row_ticket, 0, 2 * sizeof(int), st);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(w.rows, rows.data(), sizeof(RowWork) * rows.size(),
+                            cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && !tiles.empty())
+        e = cudaMemcpyAsync(w.tiles, tiles.data(), sizeof(TileWork) * tiles.size(),
+                            cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && !runs.empty())
+        e = cudaMemcpyAsync(d_runs, runs.data(), sizeof(TileRun) * runs.size(),
+                            cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess)
+        e = launch_run_tiles(b->row_ptr, d_runs, (int)runs.size(), nbounds, tile, w.tile_ptr, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    cudaFree(d_runs);
+    if (e != cudaSuccess) return e;
+    switch (b->k) {
+        case 2: batch_work_grids<2>(b->cfg.seg, &w.tiles_grid, &w.rows_grid); break;
+        case 4: batch_work_grids<4>(b->cfg.seg, &w.tiles_grid, &w.rows_grid); break;
+        default: batch_work_grids<8>(b->cfg.seg, &w.tiles_grid, &w.rows_grid); break;
+    }
+    b->mixed = w.tiles_grid > 0 && w.rows_grid > 0;
+    return cudaSuccess;
+}
+
+// Whether an execute runs the work list (else the tile kernel over the whole batch).
+static bool batch_takes_work(const bhsp_batch* b) { return b->mixed && !b->variant_set; }
 
 extern "C" int bhsp_batch_create(bhsp_batch** out, int count, int m_total, int n_total,
                                  int nnz_total, const int* d_row_ptr, const int* d_col_idx, int k,
@@ -446,6 +371,7 @@ extern "C" int bhsp_batch_create(bhsp_batch** out, int count, int m_total, int n
     if (e == cudaSuccess) e = cudaMemsetAsync(b->err, 0, sizeof(uint32_t), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->ticket, 0, 2 * sizeof(int), st);
     if (e == cudaSuccess) e = launch_partition(d_row_ptr, m_total, nnz_total, 32 * c.seg, b->tile_ptr, st);
+    if (e == cudaSuccess) e = batch_work_build(b, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
         rc = batch_cuda(b, e, "batch setup");
@@ -475,6 +401,15 @@ static BatchLaunch batch_launch(bhsp_batch* b, const float* val, const void* x, 
     return l;
 }
 
+static cudaError_t enqueue(bhsp_batch* b, const BatchLaunch& l, cudaStream_t st) {
+    if (!batch_takes_work(b)) return enqueue_batch(l, b->k, b->cfg, b->var, b->grid, st);
+    switch (b->k) {
+        case 2: return launch_batch_work<2>(l, b->work, b->cfg.seg, st);
+        case 4: return launch_batch_work<4>(l, b->work, b->cfg.seg, st);
+        default: return launch_batch_work<8>(l, b->work, b->cfg.seg, st);
+    }
+}
+
 extern "C" int bhsp_batch_execute(bhsp_batch* b, const float* d_val, const float* d_x, float* d_y,
                                   int use_graph, void* stream) {
     if (!b || !d_y || (b->nnz > 0 && (!d_val || !d_x))) return BHSPARSE_INVALID_ARGUMENT;
@@ -484,7 +419,7 @@ extern "C" int bhsp_batch_execute(bhsp_batch* b, const float* d_val, const float
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const BatchLaunch l = batch_launch(b, d_val, d_x, d_y);
     if (!use_graph) {
-        cudaError_t e = enqueue_batch(l, b->k, b->cfg, b->var, b->grid, st);
+        cudaError_t e = enqueue(b, l, st);
         return e == cudaSuccess ? BHSPARSE_SUCCESS : batch_cuda(b, e, "batched launch");
     }
     if (!b->exec || b->g_val != d_val || b->g_x != d_x || b->g_y != d_y) {
@@ -498,7 +433,7 @@ extern "C" int bhsp_batch_execute(bhsp_batch* b, const float* d_val, const float
         if (e != cudaSuccess) return batch_cuda(b, e, "capture stream");
         e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            cudaError_t e2 = enqueue_batch(l, b->k, b->cfg, b->var, b->grid, cs);
+            cudaError_t e2 = enqueue(b, l, cs);
             e = cudaStreamEndCapture(cs, &b->graph);
             if (e == cudaSuccess) e = e2;
         }
@@ -536,8 +471,9 @@ extern "C" int bhsp_batch_info(const bhsp_batch* b, int* ntiles, int* nworkers, 
     if (!b) return BHSPARSE_INVALID_ARGUMENT;
     if (ntiles) *ntiles = b->ntiles;
     if (nworkers) *nworkers = b->nworkers;
-    if (grid) *grid = b->grid;
-    if (launches) *launches = b->nworkers > 0 ? 2 : 1;
+    if (grid) *grid = batch_takes_work(b) ? b->work.rows_grid : b->grid;
+    if (launches)
+        *launches = batch_takes_work(b) ? (b->work.ntiles > 0 ? 2 : 1) : (b->nworkers > 0 ? 2 : 1);
     return BHSPARSE_SUCCESS;
 }
 
@@ -569,6 +505,7 @@ extern "C" int bhsp_batch_set_variant(bhsp_batch* b, int one_head, int l2_only) 
     if (grid <= 0) return batch_cuda(b, cudaErrorInvalidConfiguration, "batch variant");
     b->var = v;
     b->grid = grid;
+    if (one_head >= 0 || l2_only >= 0) b->variant_set = true;
     // the captured graph launches the previous kernel: capture again at the next execute
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);

@@ -57,6 +57,10 @@ struct TileArgs {
     uint32_t* err;
     int m, n, nnz;
     int phase;  // bit 0: tile kernel, bit 1: calibration kernel
+    // a window of a larger matrix (tile_worker's WIN): row_ptr and y start at the window's first
+    // row, nnz is the end of its non-zeros; slots before `begin` are padding like those from nnz on
+    int begin = 0;
+    int row0 = 0;  // the window's first row, for the carry records
     // launcher choice, made at plan time: the kernel specialised for the one-head chunk form
     // (few rows shorter than a chunk, so that most chunks take it)
     bool one_head = false;
@@ -150,29 +154,37 @@ __device__ __forceinline__ typename P::Acc warp_sum_acc(typename P::Acc v) {
 // Column indices / values of chunk c (CW non-zeros) of tile t for this lane: one vector load
 // each on full tiles, guarded scalar loads on the matrix's last, partial tile (column -1 and
 // value 0 mark padding slots, which contribute nothing and read no x).
-template <class P, int S, int CW>
+template <int TILE, bool WIN, class P>
+__device__ __forceinline__ bool full_tile(const TileArgs<P>& a, int t) {
+    return (long long)(t + 1) * TILE <= a.nnz && (!WIN || t * TILE >= a.begin);
+}
+template <bool WIN, class P>
+__device__ __forceinline__ bool real_slot(const TileArgs<P>& a, int e) {
+    return e < a.nnz && (!WIN || e >= a.begin);
+}
+template <class P, int S, int CW, bool WIN = false>
 __device__ __forceinline__ void load_cols(const TileArgs<P>& a, int t, int c, int lane,
                                           uint64_t pol, int (&cc)[CW]) {
     constexpr int TILE = 32 * S;
     const int e = t * TILE + lane * S + c * CW;
-    if ((long long)(t + 1) * TILE <= a.nnz) {
+    if (full_tile<TILE, WIN>(a, t)) {
         uint32_t u[CW];
         ld_stream_u32s(a.col + e, pol, u);
 #pragma unroll
         for (int i = 0; i < CW; ++i) cc[i] = (int)u[i];
     } else {
 #pragma unroll
-        for (int i = 0; i < CW; ++i) cc[i] = e + i < a.nnz ? a.col[e + i] : -1;
+        for (int i = 0; i < CW; ++i) cc[i] = real_slot<WIN>(a, e + i) ? a.col[e + i] : -1;
     }
 }
 // S = 8: a lane's 8 column indices of tile t (one 32-byte sector) in one load, split into the
 // tile's two 4-slot chunks.  Two 16-byte loads a chunk apart read the sector twice when the x
 // gathers in between evict it from L1.
-template <class P>
+template <bool WIN = false, class P>
 __device__ __forceinline__ void load_cols_tile8(const TileArgs<P>& a, int t, int lane, uint64_t pol,
                                                 int (&c0)[4], int (&c1)[4]) {
     const int e = t * 256 + lane * 8;
-    if ((long long)(t + 1) * 256 <= a.nnz) {
+    if (full_tile<256, WIN>(a, t)) {
         uint32_t u[8];
         ld_stream_b32x8(a.col + e, pol, u);
 #pragma unroll
@@ -183,8 +195,8 @@ __device__ __forceinline__ void load_cols_tile8(const TileArgs<P>& a, int t, int
     } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            c0[i] = e + i < a.nnz ? a.col[e + i] : -1;
-            c1[i] = e + 4 + i < a.nnz ? a.col[e + 4 + i] : -1;
+            c0[i] = real_slot<WIN>(a, e + i) ? a.col[e + i] : -1;
+            c1[i] = real_slot<WIN>(a, e + 4 + i) ? a.col[e + 4 + i] : -1;
         }
     }
 }
@@ -209,11 +221,11 @@ __device__ __forceinline__ void load_vals_full(const float* val, int e, uint64_t
 }
 // S = 8, 4-byte values: a lane's 8 values of tile t (one 32-byte sector) in one load, split into
 // the tile's two 4-slot chunks
-template <class P>
+template <bool WIN = false, class P>
 __device__ __forceinline__ void load_vals_tile8(const TileArgs<P>& a, int t, int lane, uint64_t pol,
                                                 typename P::VC (&v0)[4], typename P::VC (&v1)[4]) {
     const int e = t * 256 + lane * 8;
-    if ((long long)(t + 1) * 256 <= a.nnz) {
+    if (full_tile<256, WIN>(a, t)) {
         uint32_t u[8];
         ld_stream_b32x8(a.val + e, pol, u);
 #pragma unroll
@@ -224,8 +236,8 @@ __device__ __forceinline__ void load_vals_tile8(const TileArgs<P>& a, int t, int
     } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            v0[i] = e + i < a.nnz ? to_compute(a.val[e + i]) : typename P::VC(0);
-            v1[i] = e + 4 + i < a.nnz ? to_compute(a.val[e + 4 + i]) : typename P::VC(0);
+            v0[i] = real_slot<WIN>(a, e + i) ? to_compute(a.val[e + i]) : typename P::VC(0);
+            v1[i] = real_slot<WIN>(a, e + 4 + i) ? to_compute(a.val[e + 4 + i]) : typename P::VC(0);
         }
     }
 }
@@ -240,17 +252,17 @@ __device__ __forceinline__ void load_vals_full(const __nv_bfloat16* val, int e, 
         v[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
     }
 }
-template <class P, int S, int CW>
+template <class P, int S, int CW, bool WIN = false>
 __device__ __forceinline__ void load_vals(const TileArgs<P>& a, int t, int c, int lane,
                                           uint64_t pol, typename P::VC (&v)[CW]) {
     constexpr int TILE = 32 * S;
     const int e = t * TILE + lane * S + c * CW;
-    if ((long long)(t + 1) * TILE <= a.nnz) {
+    if (full_tile<TILE, WIN>(a, t)) {
         load_vals_full(a.val, e, pol, v);
     } else {
 #pragma unroll
         for (int i = 0; i < CW; ++i)
-            v[i] = e + i < a.nnz ? to_compute(a.val[e + i]) : typename P::VC(0);
+            v[i] = real_slot<WIN>(a, e + i) ? to_compute(a.val[e + i]) : typename P::VC(0);
     }
 }
 
@@ -344,9 +356,10 @@ __device__ __forceinline__ void chunk_segments(bool one_head, uint32_t cb, int k
 // multiplied, the values of chunk g+1 and the column indices of chunk g+2 are in flight and the
 // x gathers of chunk g+1 are issued; the bit flags' row_ptr entries and tile_ptr are fetched
 // one tile ahead.
-template <class P, int S, bool OH = false, bool MID = false, bool XL2 = false>
-__device__ __forceinline__ void tile_worker(const TileArgs<P>& a, int worker, int tpw, int ntiles,
-                                            uint32_t* const s_words_w, int* const rowof) {
+template <class P, int S, bool OH = false, bool MID = false, bool XL2 = false, bool WIN = false>
+__device__ __forceinline__ void tile_worker(const TileArgs<P>& a, int worker, int t_begin,
+                                            int t_end, uint32_t* const s_words_w,
+                                            int* const rowof) {
     using Acc = typename P::Acc;
     using Carry = typename P::Carry;
     using VC = typename P::VC;
@@ -358,8 +371,6 @@ __device__ __forceinline__ void tile_worker(const TileArgs<P>& a, int worker, in
     // the one-head chunk form (scalar accumulators only; wide ones keep the per-slot loop)
     constexpr bool one_head = OH && sizeof(Acc) <= 8;
     const int lane = threadIdx.x & 31;
-    const int t_begin = worker * tpw;
-    const int t_end = min(t_begin + tpw, ntiles);
     const uint64_t pol_s = policy_evict_first();
     const uint64_t pol_x = policy_evict_last();
 
@@ -377,15 +388,15 @@ __device__ __forceinline__ void tile_worker(const TileArgs<P>& a, int worker, in
     VC valC[CW] = {};
     {
         int col0[CW];
-        load_cols<P, S, CW>(a, t_begin, 0, lane, pol_s, col0);
+        load_cols<P, S, CW, WIN>(a, t_begin, 0, lane, pol_s, col0);
         if constexpr (whole_val_sector)
-            load_vals_tile8(a, t_begin, lane, pol_s, valA, valC);
+            load_vals_tile8<WIN>(a, t_begin, lane, pol_s, valA, valC);
         else
-            load_vals<P, S, CW>(a, t_begin, 0, lane, pol_s, valA);
+            load_vals<P, S, CW, WIN>(a, t_begin, 0, lane, pol_s, valA);
         gather_cw<XL2>(a.x, col0, pol_x, xA);
         const int t1 = t_begin + (NC > 1 ? 0 : 1);
         const int c1 = NC > 1 ? 1 : 0;
-        if (t1 < t_end) load_cols<P, S, CW>(a, t1, c1, lane, pol_s, colA);
+        if (t1 < t_end) load_cols<P, S, CW, WIN>(a, t1, c1, lane, pol_s, colA);
     }
 
     int carry_row = -1;  // row of the segment left open by the previous tile (-1: none)
@@ -399,7 +410,7 @@ __device__ __forceinline__ void tile_worker(const TileArgs<P>& a, int worker, in
             if (owned) {
                 store_row(a.y, a.m, row, P::out_carry(v), a.err);
             } else {
-                a.rec_row[worker] = row;
+                a.rec_row[worker] = WIN ? a.row0 + row : row;
                 a.rec_val[worker] = P::rec_from(v);
             }
         }
@@ -485,13 +496,13 @@ __device__ __forceinline__ void tile_worker(const TileArgs<P>& a, int worker, in
             const int t2 = t + (c + 2) / NC, c2 = (c + 2) % NC;
             if constexpr (whole_col_sector) {
                 if (c == 0) {  // the next tile's columns, both chunks
-                    if (t + 1 < t_end) load_cols_tile8(a, t + 1, lane, pol_s, colB, colC);
+                    if (t + 1 < t_end) load_cols_tile8<WIN>(a, t + 1, lane, pol_s, colB, colC);
                 } else {
 #pragma unroll
                     for (int k = 0; k < CW; ++k) colB[k] = colC[k];
                 }
             } else {
-                if (t2 < t_end) load_cols<P, S, CW>(a, t2, c2, lane, pol_s, colB);
+                if (t2 < t_end) load_cols<P, S, CW, WIN>(a, t2, c2, lane, pol_s, colB);
             }
             if (t1 < t_end) {
                 if constexpr (whole_val_sector) {
@@ -499,14 +510,14 @@ __device__ __forceinline__ void tile_worker(const TileArgs<P>& a, int worker, in
 #pragma unroll
                         for (int k = 0; k < CW; ++k) valB[k] = valC[k];
                     } else {  // the next tile's values, both chunks
-                        load_vals_tile8(a, t1, lane, pol_s, valB, valC);
+                        load_vals_tile8<WIN>(a, t1, lane, pol_s, valB, valC);
                     }
                 } else {
-                    load_vals<P, S, CW>(a, t1, c1, lane, pol_s, valB);
+                    load_vals<P, S, CW, WIN>(a, t1, c1, lane, pol_s, valB);
                 }
                 // the one-head kernels gather a full tile's x without the padding test (1 %
                 // on the 27-point stencil; the per-slot kernels measured no gain from it)
-                if (one_head && (long long)(t1 + 1) * TILE <= a.nnz)
+                if (one_head && full_tile<TILE, WIN>(a, t1))
                     gather_cw_full<XL2>(a.x, colA, pol_x, xB);
                 else
                     gather_cw<XL2>(a.x, colA, pol_x, xB);
@@ -623,7 +634,8 @@ __global__ void __launch_bounds__(WARPS * 32, (resident_warps<P, S, OH>() / WARP
     const int warp = threadIdx.x >> 5;
     const int worker = blockIdx.x * WARPS + warp;
     if (worker >= nworkers) return;
-    tile_worker<P, S, OH, MID, XL2>(a, worker, tpw, ntiles, s_words[warp], s_rowof[warp]);
+    tile_worker<P, S, OH, MID, XL2>(a, worker, worker * tpw, min((worker + 1) * tpw, ntiles),
+                                    s_words[warp], s_rowof[warp]);
 }
 
 // Persistent tile kernels: a grid of at most the GPU's resident capacity in which each warp takes
@@ -649,7 +661,8 @@ __device__ __forceinline__ void persistent_workers(const TileArgs<P>& a, int tpw
             if (lane == 0) atomicOr(a.err, ERR_QUEUE);
             break;
         }
-        tile_worker<P, S, OH, MID, XL2>(a, w, tpw, ntiles, s_words_w, rowof);
+        tile_worker<P, S, OH, MID, XL2>(a, w, w * tpw, min((w + 1) * tpw, ntiles), s_words_w,
+                                        rowof);
         __syncwarp();
     }
     if (lane == 0) {
@@ -753,56 +766,65 @@ __device__ __forceinline__ R rec_shfl_xor(const R& v, int d) {
 // spans several workers) forms a contiguous run; the warp that holds the run's first record sums
 // it cooperatively: lanes take records 32 apart, then a butterfly reduction, so a run of L
 // records costs ceil(L/32) rounds instead of L dependent loads, in an order fixed by L alone
-// (deterministic).  Also zeroes the leading empty rows, which lie in no tile span (the
-// reference never writes them).
+// (deterministic).
+template <class P>
+__device__ __forceinline__ void calibrate_records(const int* __restrict__ rec_row,
+                                                  const typename P::Rec* __restrict__ rec_val,
+                                                  int nworkers, int base,
+                                                  typename P::YT* __restrict__ y, int m,
+                                                  uint32_t* err) {
+    using Rec = typename P::Rec;
+    using YT = typename P::YT;
+    const int lane = threadIdx.x & 31;
+    const int w = base + lane;
+    const int r = w < nworkers ? rec_row[w] : -1;
+    const int rprev = (w > 0 && w < nworkers) ? rec_row[w - 1] : -1;
+    const int rnext = w + 1 < nworkers ? rec_row[w + 1] : -1;
+    const bool head = r >= 0 && rprev != r;
+    const bool single = head && rnext != r;
+    if (single) {
+        if (r < m)
+            y[r] = P::out_rec(P::rec_add(P::rec_of_y(y[r]), rec_val[w]));
+        else
+            atomicOr(err, ERR_BAD_TILE);
+    }
+    unsigned runs = __ballot_sync(SPMV_FULL_MASK, head && !single);
+    while (runs) {
+        const int src = __ffs(runs) - 1;
+        runs &= runs - 1;
+        const int w0 = base + src;
+        const int row = __shfl_sync(SPMV_FULL_MASK, r, src);
+        Rec acc = P::rec_of_y(YT(0));
+        for (int v = w0 + lane;; v += 32) {
+            const bool in = v < nworkers && rec_row[v] == row;
+            if (in) acc = P::rec_add(acc, rec_val[v]);
+            if (__ballot_sync(SPMV_FULL_MASK, in) != SPMV_FULL_MASK) break;  // the run ended
+        }
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) acc = P::rec_add(acc, rec_shfl_xor(acc, d));
+        if (lane == 0) {
+            if (row < m)
+                y[row] = P::out_rec(P::rec_add(P::rec_of_y(y[row]), acc));
+            else
+                atomicOr(err, ERR_BAD_TILE);
+        }
+    }
+}
+
+// Also zeroes the leading empty rows, which lie in no tile span (the reference never writes them).
 template <class P>
 __global__ void k_calibrate(const int* __restrict__ rec_row,
                             const typename P::Rec* __restrict__ rec_val, int nworkers,
                             typename P::YT* __restrict__ y, const uint32_t* __restrict__ tile_ptr,
                             int m, uint32_t* err) {
-    using Rec = typename P::Rec;
     using YT = typename P::YT;
     // launched as a programmatic dependent of the tile kernel: wait until that grid has
     // completed and its records and y are visible (returns at once for an ordinary launch)
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int lane = threadIdx.x & 31;
     const int nwarps = gridDim.x * (blockDim.x >> 5);
     const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    for (int base = gw * 32; base < nworkers; base += nwarps * 32) {  // warp-uniform
-        const int w = base + lane;
-        const int r = w < nworkers ? rec_row[w] : -1;
-        const int rprev = (w > 0 && w < nworkers) ? rec_row[w - 1] : -1;
-        const int rnext = w + 1 < nworkers ? rec_row[w + 1] : -1;
-        const bool head = r >= 0 && rprev != r;
-        const bool single = head && rnext != r;
-        if (single) {
-            if (r < m)
-                y[r] = P::out_rec(P::rec_add(P::rec_of_y(y[r]), rec_val[w]));
-            else
-                atomicOr(err, ERR_BAD_TILE);
-        }
-        unsigned runs = __ballot_sync(SPMV_FULL_MASK, head && !single);
-        while (runs) {
-            const int src = __ffs(runs) - 1;
-            runs &= runs - 1;
-            const int w0 = base + src;
-            const int row = __shfl_sync(SPMV_FULL_MASK, r, src);
-            Rec acc = P::rec_of_y(YT(0));
-            for (int v = w0 + lane;; v += 32) {
-                const bool in = v < nworkers && rec_row[v] == row;
-                if (in) acc = P::rec_add(acc, rec_val[v]);
-                if (__ballot_sync(SPMV_FULL_MASK, in) != SPMV_FULL_MASK) break;  // the run ended
-            }
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) acc = P::rec_add(acc, rec_shfl_xor(acc, d));
-            if (lane == 0) {
-                if (row < m)
-                    y[row] = P::out_rec(P::rec_add(P::rec_of_y(y[row]), acc));
-                else
-                    atomicOr(err, ERR_BAD_TILE);
-            }
-        }
-    }
+    for (int base = gw * 32; base < nworkers; base += nwarps * 32)  // warp-uniform
+        calibrate_records<P>(rec_row, rec_val, nworkers, base, y, m, err);
     const long long stride = (long long)gridDim.x * blockDim.x;
     const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const int lead = min((int)(tile_ptr[0] & ROW_MASK), m);

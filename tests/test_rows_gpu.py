@@ -126,3 +126,66 @@ def test_row_kernel_decision(cuda_ok):
     assert launches(uneven) == 2
     three_quarters = rng.integers(20, 28, m)  # 24 of 28 slots on average
     assert launches(three_quarters) == 1
+
+
+@pytest.mark.parametrize("k", [2, 4, 8])
+@pytest.mark.parametrize("seg", [8, 16, 32])
+def test_batch_work_lists_bit_exact(cuda_ok, k, seg):
+    """The batched form's row and tile workers in one batch: runs of long rows that begin and end
+    inside a tile, between blocks of every row layout; empty rows at the start and end of a run
+    and of the batch, an all-empty member, a last block of a few rows, non-zeros not a multiple of
+    8; run twice, and against the one tile kernel (a forced variant)."""
+    import torch
+    from benchmark_spmv_using_csr_gb300 import batch, gen
+    rng = np.random.default_rng(10 * k + seg)
+
+    def rows(lens):
+        a = gen.from_row_lengths(np.asarray(lens), 3000, seed=int(rng.integers(1 << 30)))
+        a.val = rng.integers(-4, 5, a.nnz).astype(np.float64)
+        return a
+
+    long_rows = rng.integers(0, 40, 700)
+    long_rows[[5, 300, 690]] = [2500, 225, 1111]
+    long_rows[:4] = long_rows[-3:] = 0
+    mats = [rows(np.zeros(300, int)), rows(np.full(513, 27)), rows(long_rows),
+            rows(np.full(260, 32)), rows(np.full(1024, 5)), rows(rng.integers(50, 57, 256)),
+            rows(long_rows[::-1]), rows(rng.integers(100, 113, 256)),
+            rows(rng.integers(200, 225, 256)), rows(np.full(3, 7))]
+    b = batch.Batch(mats, k=k, seg=seg)
+    info = b.info()
+    assert info["launches"] == 2
+    x_np = rng.integers(-4, 5, (b.n, k)).astype(np.float64)
+    cat = b.cat
+    row = np.repeat(np.arange(b.m), np.diff(cat["row_ptr"]))
+    want = np.zeros((b.m, k))
+    np.add.at(want, row, cat["val"][:, None] * x_np[cat["col"]])
+    x = torch.from_numpy(x_np.astype(np.float32)).cuda()
+    y = torch.empty((b.m, k), dtype=torch.float32, device="cuda")
+    grids = set()
+    for l2 in (None, None, True):
+        b.set_variant(l2_only=l2)
+        grids.add(b.info()["grid"])
+        for use_graph in (True, False):
+            y.fill_(float("nan"))
+            b.execute(x, y, use_graph=use_graph)
+            b.check()
+            assert (y.cpu().numpy() == want).all(), (l2, use_graph)
+    b.close()
+
+
+def test_batch_of_regular_members_is_one_launch(cuda_ok):
+    """No run of long rows: no tile workers and no carry records."""
+    import torch
+    from benchmark_spmv_using_csr_gb300 import batch, gen
+    a = gen.stencil3d(20, 21, 22, seed=3)
+    a.val = gen.uniform_int(a.nnz, 8, 10) - 4.0
+    b = batch.Batch([a, a], k=4)
+    assert b.info()["launches"] == 1
+    x = torch.ones((b.n, 4), dtype=torch.float32, device="cuda")
+    y = torch.full((b.m, 4), float("nan"), dtype=torch.float32, device="cuda")
+    b.execute(x, y)
+    b.check()
+    row = np.repeat(np.arange(a.m), np.diff(a.row_ptr))
+    want = np.bincount(row, a.val, a.m)
+    assert (y.cpu().numpy() == np.tile(want, 2)[:, None]).all()
+    b.close()
