@@ -300,24 +300,28 @@ cudaError_t launch_run_tiles(const int* row_ptr, const TileRun* runs, int nruns,
 }
 
 // Whether a matrix takes the row kernel, and with which lane layout.
-//  * Columns with locality (x_l2 false): lanes on rows pay through coalesced x reads, which random
-//    columns do not have (a power-law or uniform-density matrix ran 1.2-4x slower here).
 //  * The longest row fits in T = 8 lanes of 28 slots (224 non-zeros), FP64 in 32 non-zeros: its
 //    slots beyond the row's end cost as much of the narrow FP64 pipe as real ones, and with 2 or
 //    more lanes to a row it was 0.86-1.1x the tile kernel.
-//  * The rows fill the slots that their pass walks.  Measured against the tile kernel at the best
-//    of six schedules on banded matrices of 1e6-4e7 non-zeros (time tile / time rows): from a
-//    share of 0.6 on 0.97-1.8x in FP32, 0.97-1.7x in mixed FP32, 1.1-2.0x in BF16 storage (0.5
-//    and below: 0.87-1.2x); in FP64 with rows of up to 12 non-zeros 1.1-1.9x, with longer ones
-//    1.0-1.5x from 0.84 on and 0.73-0.98x below.
+//  * The rows fill a share of the slots that their passes walk.  Measured against the tile kernel at
+//    the best of six schedules (time tile / time rows), by value type and columns:
+//    - 4- and 2-byte values, near columns (banded matrices of 1e6-4e7 non-zeros): from a share of
+//      0.6 on 0.97-2.0x, at 0.5 and below 0.87-1.2x;
+//    - 4- and 2-byte values, random columns (Poisson and constant rows, 2e6-6e7 non-zeros): from
+//      0.35 on 1.01-2.4x (1.2x at 8e6), at 0.2-0.3 0.88-1.5x.  The threshold is lower because the
+//      tile kernel's gathers wait in turn where a pass has all of its own in flight;
+//    - FP64, rows of up to 12 non-zeros, near columns: 1.1-1.9x from 0.6 on;
+//    - FP64 else: 1.0-1.5x from 0.84 on, 0.58-0.98x below (Poisson rows: the longest of 32 rows is
+//      twice the mean, and so is the FP64 pipe's time).
 RowForm choose_row_form(const RowCounts& c, int m, int nnz, bool x_l2, bool f64) {
     RowForm f;
     // the kernel counts rows in whole passes of 32: their numbers must not pass 2^31
-    if (x_l2 || nnz == 0 || m > 0x7fffff00 || c.max_len > (f64 ? 32u : 224u)) return f;
+    if (nnz == 0 || m > 0x7fffff00 || c.max_len > (f64 ? 32u : 224u)) return f;
     int t = 0;  // log2 of the lanes per row
     while (c.max_len > (28ull << t)) ++t;
     const double slots = 128.0 * (double)c.groups[t];
-    if ((double)nnz < (f64 && c.max_len > 12 ? 0.84 : 0.6) * slots) return f;
+    const double share = f64 ? (x_l2 || c.max_len > 12 ? 0.84 : 0.6) : x_l2 ? 0.33 : 0.6;
+    if ((double)nnz < share * slots) return f;
     f.lanes = 1 << t;
     f.groups = (int)((c.max_len + (4u << t) - 1) >> (2 + t));
     f.rotate = 2 * c.eights > (unsigned long long)m;

@@ -1,4 +1,4 @@
-// row_kernel.cuh -- y = A.x for matrices whose rows are short and of much the same length, with
+// row_kernel.cuh -- y = A.x for matrices whose rows are short and fill their lanes' slots, with
 // lanes assigned to whole rows; generic over the arithmetic policies of tile_kernel.cuh.
 //
 // A pass is 32 / T consecutive rows, T lanes to a row (T = 1, 2, 4 or 8).  The pass's stretch of
@@ -18,6 +18,10 @@
 // the FP64 pipe needs 195 us for its 28 slots a row, memory 208 us); BF16 storage on 121 x 97 x
 // 143 86 -> 49.5 us (5800 GB/s); the 5-point stencil on 256^2, FP64, 8.7 -> 7.2 us (the host's
 // launch path).
+//
+// Random columns: Poisson rows of 8, 8 M non-zeros, mixed FP32 46 -> 38 us (a gather's sector per
+// slot: 227 G/s, the L2-to-SM rate for random sectors being 290-320); read from L2 only they are
+// 1-2 % faster above 5e7 non-zeros and up to 20 % slower below, so they allocate in L1.
 //
 // What bounds it: bytes in flight.  The stage is free once it has been read into registers, so
 // the next pass's copies run during this pass's gathers and multiply-adds, and 16-40 warps per SM
@@ -248,14 +252,25 @@ __global__ void __launch_bounds__(ROW_WARPS * 32, (row_min_ctas<P, NG>())) k_row
             }
         }
         fill_stage();
-        Acc acc = P::zero();
+        // plain FP32 sums in 4 parts, so that the chains of roundings are no longer than the tile
+        // kernel's (one part: 1.16x its error on Poisson rows of 20; 4 parts: 0.85x)
+        constexpr int NP = std::is_same<Acc, float>::value ? 4 : 1;
+        Acc part[NP];
+#pragma unroll
+        for (int i = 0; i < NP; ++i) part[i] = P::zero();
 #pragma unroll
         for (int g = 0; g < U; g += 4) {
             if (g * T < top) {
 #pragma unroll
-                for (int u = g; u < g + 4; ++u) acc = P::fma(v[u], x[u], acc);
+                for (int u = g; u < g + 4; ++u) part[u % NP] = P::fma(v[u], x[u], part[u % NP]);
             }
         }
+#pragma unroll
+        for (int d = 1; d < NP; d <<= 1) {
+#pragma unroll
+            for (int i = 0; i < NP; i += 2 * d) part[i] = P::add(part[i], part[i + d]);
+        }
+        Acc acc = part[0];
 #pragma unroll
         for (int d = 1; d < T; d <<= 1) acc = P::add(acc, sh_xor(acc, d));
         if (j == 0 && my_row < a.m) a.y[my_row] = P::out_acc(acc);

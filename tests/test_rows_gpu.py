@@ -1,5 +1,5 @@
 """The row kernel (lanes assigned to whole rows), which a plan takes for matrices whose rows are
-short, of much the same length and with columns of some locality: bit for bit against an int64
+short and fill their lanes' slots: bit for bit against an int64
 sum on integer-valued data, at the edges of its lane layouts (1 to 8 lanes per row, 1 to 7 groups
 of 4 slots each), of its passes of 32 lanes and of the bulk copies' groups of 8 non-zeros."""
 import numpy as np
@@ -99,8 +99,8 @@ def test_many_passes_per_warp_bit_exact(cuda_ok, vt):
 
 
 def test_row_kernel_decision(cuda_ok):
-    """Short rows of one length with near columns take the row kernel; random columns, one long
-    row, and rows that would leave most slots empty do not."""
+    """Short rows that fill their slots take the row kernel: 0.6 of them with near columns, a third
+    with random ones, 0.84 in FP64; one long row sends the matrix to the tile kernels."""
     import torch
     rng = np.random.default_rng(1)
 
@@ -117,13 +117,14 @@ def test_row_kernel_decision(cuda_ok):
     m = 20_000
     whole = np.full(m, 27)
     assert launches(whole) == 1 and launches(whole, sp.VALUE_F64) == 1
-    assert launches(whole, spread=True) == 2
+    assert launches(whole, spread=True) == 1 and launches(whole, sp.VALUE_F64, spread=True) == 1
     one_long = whole.copy()
     one_long[77] = 225
     assert launches(one_long) == 2
     assert launches(np.full(m, 33), sp.VALUE_F64) == 2 and launches(np.full(m, 33)) == 1
-    uneven = rng.integers(0, 28, m)
-    assert launches(uneven) == 2
+    uneven = rng.integers(0, 28, m)  # half of the 28 slots on average
+    assert launches(uneven) == 2 and launches(uneven, spread=True) == 1
+    assert launches(uneven, sp.VALUE_F64, spread=True) == 2
     three_quarters = rng.integers(20, 28, m)  # 24 of 28 slots on average
     assert launches(three_quarters) == 1
 
