@@ -748,25 +748,32 @@ void launch_tile_kernel(const TileArgs<P>& a, int tpw, int nworkers, int ntiles,
 }
 
 // Exchange of any carry-record type between lanes (as 32-bit words).
-template <class R>
-__device__ __forceinline__ R rec_shfl_xor(const R& v, int d) {
+template <bool DOWN, class R>
+__device__ __forceinline__ R rec_shfl(const R& v, int d) {
     static_assert(sizeof(R) % 4 == 0, "records are whole 32-bit words");
     constexpr int W = (int)(sizeof(R) / 4);
     uint32_t w[W];
     memcpy(w, &v, sizeof(R));
 #pragma unroll
-    for (int i = 0; i < W; ++i) w[i] = __shfl_xor_sync(SPMV_FULL_MASK, w[i], d);
+    for (int i = 0; i < W; ++i)
+        w[i] = DOWN ? __shfl_down_sync(SPMV_FULL_MASK, w[i], d)
+                    : __shfl_xor_sync(SPMV_FULL_MASK, w[i], d);
     R r;
     memcpy(&r, w, sizeof(R));
     return r;
 }
 
-// Carry records -> y.  One warp per 32 consecutive records.  A record whose row has no other
-// record (the common case) is added by its own lane.  A row with several records (a row that
-// spans several workers) forms a contiguous run; the warp that holds the run's first record sums
-// it cooperatively: lanes take records 32 apart, then a butterfly reduction, so a run of L
-// records costs ceil(L/32) rounds instead of L dependent loads, in an order fixed by L alone
+// Carry records -> y.  One warp per 32 consecutive records.  A row with several records (a row that
+// spans several workers) forms a contiguous run of them.  The runs that lie within a warp's 32 are
+// summed by shuffles, all at once; the one run that may leave the warp is summed to its end by the
+// warp that holds its first record.  The order of every sum is fixed by the records' places alone
 // (deterministic).
+// Bound by the latency of its few dependent loads, which nothing hides: the rows and the records
+// come in one round, and a run behind the warp U records a lane at a time.  One round per
+// dependent load, as it was (rows, neighbours, records, 32 records of a run at a time), cost the
+// dense-row matrix of 1M rows 61.2 us per product in FP64 where it now takes 58.8, the power-law
+// matrix of 700K rows 61.3 -> 57.9 (mixed FP32), and, at 256 non-zeros per worker (4000 records in
+// the longest run), 114 -> 62 us.
 template <class P>
 __device__ __forceinline__ void calibrate_records(const int* __restrict__ rec_row,
                                                   const typename P::Rec* __restrict__ rec_val,
@@ -777,37 +784,65 @@ __device__ __forceinline__ void calibrate_records(const int* __restrict__ rec_ro
     using YT = typename P::YT;
     const int lane = threadIdx.x & 31;
     const int w = base + lane;
+    // The records, their rows and the two rows beside the warp's 32, all in one round of loads.
     const int r = w < nworkers ? rec_row[w] : -1;
-    const int rprev = (w > 0 && w < nworkers) ? rec_row[w - 1] : -1;
-    const int rnext = w + 1 < nworkers ? rec_row[w + 1] : -1;
+    const int edge = lane == 0 ? base - 1 : base + 32;
+    const int re = (lane == 0 || lane == 31) && edge >= 0 && edge < nworkers ? rec_row[edge] : -1;
+    const Rec none = P::rec_of_y(YT(0));
+    Rec acc = none;
+    if (r >= 0) acc = rec_val[w];
+    int rprev = __shfl_up_sync(SPMV_FULL_MASK, r, 1);
+    int rnext = __shfl_down_sync(SPMV_FULL_MASK, r, 1);
+    if (lane == 0) rprev = re;
+    if (lane == 31) rnext = re;
     const bool head = r >= 0 && rprev != r;
-    const bool single = head && rnext != r;
-    if (single) {
+    const bool far = r >= 0 && rnext == r;  // the run goes on behind this record
+    if (__any_sync(SPMV_FULL_MASK, far)) {
+        // Runs of several records: a run lies in neighbouring lanes, so five steps leave in its
+        // first lane the sum of all its records in this warp.
+        const bool goes_on = __shfl_sync(SPMV_FULL_MASK, (int)far, 31);
+        const int last = __shfl_sync(SPMV_FULL_MASK, r, 31);
+        const unsigned starts = __ballot_sync(SPMV_FULL_MASK, head && r == last);
+        Rec own = r == last ? acc : none;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const Rec o = rec_shfl<true>(acc, d);
+            const int ro = __shfl_down_sync(SPMV_FULL_MASK, r, d);
+            if (lane + d < 32 && ro == r) acc = P::rec_add(acc, o);
+        }
+        if (goes_on && starts) {
+            // The last run leaves the warp: its first warp adds it to the end, U records per lane
+            // with their loads in flight together. One round at a time it is a chain of dependent
+            // loads, about 1 us per 32 records.
+            constexpr int U = sizeof(Rec) <= 8 ? 8 : 2;
+            for (int v = base + 32 + lane;; v += 32 * U) {
+                int rr[U];
+                Rec rv[U];
+#pragma unroll
+                for (int i = 0; i < U; ++i) {
+                    const bool there = v + 32 * i < nworkers;
+                    rr[i] = there ? rec_row[v + 32 * i] : -1;
+                    rv[i] = none;
+                    if (there) rv[i] = rec_val[v + 32 * i];
+                }
+                bool all = true;
+#pragma unroll
+                for (int i = 0; i < U; ++i) {
+                    if (rr[i] == last) own = P::rec_add(own, rv[i]);
+                    all = all && rr[i] == last;
+                }
+                if (!__all_sync(SPMV_FULL_MASK, all)) break;  // the run ended
+            }
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) own = P::rec_add(own, rec_shfl<false>(own, d));
+            if (r == last) acc = own;
+        }
+    }
+    if (head) {
         if (r < m)
-            y[r] = P::out_rec(P::rec_add(P::rec_of_y(y[r]), rec_val[w]));
+            y[r] = P::out_rec(P::rec_add(P::rec_of_y(y[r]), acc));
         else
             atomicOr(err, ERR_BAD_TILE);
-    }
-    unsigned runs = __ballot_sync(SPMV_FULL_MASK, head && !single);
-    while (runs) {
-        const int src = __ffs(runs) - 1;
-        runs &= runs - 1;
-        const int w0 = base + src;
-        const int row = __shfl_sync(SPMV_FULL_MASK, r, src);
-        Rec acc = P::rec_of_y(YT(0));
-        for (int v = w0 + lane;; v += 32) {
-            const bool in = v < nworkers && rec_row[v] == row;
-            if (in) acc = P::rec_add(acc, rec_val[v]);
-            if (__ballot_sync(SPMV_FULL_MASK, in) != SPMV_FULL_MASK) break;  // the run ended
-        }
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) acc = P::rec_add(acc, rec_shfl_xor(acc, d));
-        if (lane == 0) {
-            if (row < m)
-                y[row] = P::out_rec(P::rec_add(P::rec_of_y(y[row]), acc));
-            else
-                atomicOr(err, ERR_BAD_TILE);
-        }
     }
 }
 
