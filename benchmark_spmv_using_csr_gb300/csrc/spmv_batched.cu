@@ -183,6 +183,19 @@ static int batch_cuda(bhsp_batch* b, cudaError_t e, const char* what) {
     return e == cudaErrorMemoryAllocation ? BHSPARSE_OUT_OF_MEMORY : BHSPARSE_CUDA_ERROR;
 }
 
+// The default tiles per worker.  A longer worker saves a start and a carry record per tile and
+// leaves fewer workers to even out the warps' last ones, so it is worth its length only where
+// every resident warp has many tiles.  Measured at one right-hand side and 16 non-zeros per lane
+// with 1, 2, 3 and 4 tiles (us): 2 matrices (0.7 tiles per warp) 13.5, 16.6, 18.7, 21.8; 5 (1.8)
+// 27.5, 37.1, 46.6, 57.8; 32 (12) 71, 76, 84, 98; 128 (47) 257, 229, 220, 231; 256 (90) 460, 402,
+// 394, 387.  Power-law matrices at 8 right-hand sides: 26 tiles per warp 344, 314, 311, 313.
+static int batch_tiles_per_worker(const bhsp_batch* b) {
+    const long long warps = (long long)b->grid * b->cfg.warps_per_cta;
+    int tpw = 1;
+    while (tpw < 4 && b->ntiles >= (7LL << tpw) * warps) ++tpw;
+    return tpw;
+}
+
 // The batch's work lists (see batch_kernel.cuh), from two right-hand sides on: row workers for the
 // blocks of 256 rows that suit lanes on whole rows, tile workers for the runs between them.  Leaves
 // b->mixed false where the row workers would hold less than a quarter of the batch.
@@ -315,7 +328,7 @@ extern "C" int bhsp_batch_create(bhsp_batch** out, int count, int m_total, int n
     TileConfig c;
     // default schedule: S = 16, except S = 32 for 4 right-hand sides (+1.7 % on the batched workload)
     c.seg = seg > 0 ? seg : (k == 4 ? 32 : 16);
-    c.tiles_per_worker = tiles_per_worker > 0 ? tiles_per_worker : 4;
+    c.tiles_per_worker = tiles_per_worker > 0 ? tiles_per_worker : 1;  // 0: chosen below
     c.warps_per_cta = warps_per_cta > 0 ? warps_per_cta : 4;
     c.stages = 0;
     if ((c.seg != 8 && c.seg != 16 && c.seg != 32) || (c.warps_per_cta != 4 && c.warps_per_cta != 8))
@@ -334,7 +347,6 @@ extern "C" int bhsp_batch_create(bhsp_batch** out, int count, int m_total, int n
     b->row_ptr = d_row_ptr;
     b->col = d_col_idx;
     b->ntiles = num_tiles(nnz_total, 32 * c.seg);
-    b->nworkers = (b->ntiles + c.tiles_per_worker - 1) / c.tiles_per_worker;
     cudaError_t e = cudaSuccess;
     {
         // the kernel variant, as for a single matrix's plan: short rows against the chunk
@@ -361,8 +373,10 @@ extern "C" int bhsp_batch_create(bhsp_batch** out, int count, int m_total, int n
         b->var.x_l2 = x_l2_pays(h.locality[0], h.locality[1]);
     }
     b->grid = e == cudaSuccess ? batch_grid(k, c, b->var) : 0;
-    const size_t nw = b->nworkers > 0 ? (size_t)b->nworkers : 1;
     if (e == cudaSuccess && b->grid <= 0) e = cudaErrorInvalidConfiguration;
+    if (tiles_per_worker <= 0) b->cfg.tiles_per_worker = c.tiles_per_worker = batch_tiles_per_worker(b);
+    b->nworkers = (b->ntiles + c.tiles_per_worker - 1) / c.tiles_per_worker;
+    const size_t nw = b->nworkers > 0 ? (size_t)b->nworkers : 1;
     if (e == cudaSuccess) e = cudaMalloc(&b->tile_ptr, sizeof(uint32_t) * ((size_t)b->ntiles + 1));
     if (e == cudaSuccess) e = cudaMalloc(&b->rec_row, sizeof(int) * nw);
     if (e == cudaSuccess) e = cudaMalloc(&b->rec_val, sizeof(double) * k * nw);
