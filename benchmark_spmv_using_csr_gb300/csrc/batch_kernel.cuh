@@ -1,4 +1,5 @@
-// batch_kernel.cuh -- the batched form's two kernels over work lists.
+// batch_kernel.cuh -- the batched form's two kernels over work lists (at one right-hand side the
+// row workers' is another one, batch_k1.cu).
 //
 // The matrices of a batch differ in structure, so no one kernel suits the concatenated matrix.
 // Blocks of 256 rows whose rows are short, even and local are cut into row workers (lanes on whole

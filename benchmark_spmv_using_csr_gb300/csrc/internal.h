@@ -81,7 +81,14 @@ struct RowLaunch {
     uint32_t* err;
     int m, nnz;
     RowForm form;
+    // over a list of blocks of BATCH_BLOCK rows (launch_rows_listed); `dependent`: on the kernel
+    // launched just before on the stream, another one of the same batch
+    const int* blocks = nullptr;
+    int nblocks = 0;
+    bool dependent = false;
 };
+constexpr int BATCH_BLOCK = 256;
+cudaError_t launch_rows_listed(const RowLaunch& l, cudaStream_t st);  // batch_k1.cu
 cudaError_t launch_rows_f64(const RowLaunch& l, cudaStream_t st);
 cudaError_t launch_rows_f32(const RowLaunch& l, cudaStream_t st);
 cudaError_t launch_rows_mixed_f32(const RowLaunch& l, cudaStream_t st);
@@ -164,10 +171,25 @@ struct TileWork {
     int first, last, row0, row1, at;
 };
 constexpr int BATCH_SLOTS = 28;  // of a lane in a pass: rows of up to 28, 56, 112, 224 non-zeros
+// One right-hand side: the blocks whose rows one lane layout of the row kernel takes.
+struct RowList {
+    RowForm form;
+    int first, count;  // blocks[first ...]
+};
+// lane layouts of the row lists, smaller ones first: lanes per row, groups of 4 slots per lane, and
+// the layout that takes its blocks too where they are too few for a kernel of their own (-1: none)
+struct ListForm {
+    int lanes, groups, into;
+};
+constexpr ListForm LIST_FORMS[] = {{1, 2, 1}, {1, 4, 2}, {1, 7, -1}, {2, 4, 4}, {2, 7, -1}, {4, 7, -1}};
+constexpr int NLIST_FORMS = sizeof(LIST_FORMS) / sizeof(LIST_FORMS[0]);
 // The two work lists and their kernels' buffers.
 struct BatchWork {
     TileWork* tiles = nullptr;  // [ntiles]
     RowWork* rows = nullptr;    // [nrows], the carry records' workers last
+    int* blocks = nullptr;      // one right-hand side: first rows of blocks, list by list
+    RowList lists[NLIST_FORMS];
+    int nlists = 0;
     uint32_t* tile_ptr = nullptr;
     int* rec_row = nullptr;     // [ntiles]
     void* rec_val = nullptr;
@@ -182,7 +204,6 @@ struct BlockStat {
     int eights;     // non-empty rows of a multiple of 8 non-zeros
     int filled;     // non-empty rows
 };
-constexpr int BATCH_BLOCK = 256;
 cudaError_t launch_block_stats(const int* row_ptr, int m, BlockStat* stat, cudaStream_t st);
 // A run of rows for the tile workers: tiles [t0, t1], boundary t at tile_ptr[at + t - t0].
 struct TileRun {

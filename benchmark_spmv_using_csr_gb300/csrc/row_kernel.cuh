@@ -48,6 +48,7 @@ struct RowArgs {
     int m, nnz;
     int npasses, ppw, nworkers;  // a worker is ppw consecutive passes
     bool rotate, by_ticket;
+    const int* __restrict__ blocks;  // the first rows of the blocks of 256 rows to do (LIST)
 };
 
 // one x entry where `on`, 0 elsewhere (the load is predicated: an absent slot reads nothing)
@@ -96,8 +97,12 @@ constexpr bool row_ticket_pays() {
     return sizeof(typename P::VS) == 8 && NG >= 3;
 }
 
-template <class P, int T, int NG>
+// LIST: the rows are those of a list of blocks, one kernel of several in a row for a batch.  Each
+// may start while the one before it drains and waits for that one before it ends, so that the last
+// one's end is the end of all.
+template <class P, int T, int NG, bool LIST>
 __global__ void __launch_bounds__(ROW_WARPS * 32, (row_min_ctas<P, NG>())) k_rows(RowArgs<P> a) {
+    if constexpr (LIST) asm volatile("griddepcontrol.launch_dependents;");
     using L = RowStage<P, NG>;
     using VS = typename P::VS;
     using VC = typename P::VC;
@@ -125,12 +130,19 @@ __global__ void __launch_bounds__(ROW_WARPS * 32, (row_min_ctas<P, NG>())) k_row
     // drawn one worker ahead of its use (lane 0 holds the number).
     const bool queue = row_ticket_pays<P, NG>() && a.by_ticket;
     int w = blockIdx.x * ROW_WARPS + warp;
+    constexpr int BLOCK_PASSES = BATCH_BLOCK / R;
+    int nblock = 0, base = 0;  // LIST: the first row of worker w's block; of pass 0 were it there
+    auto find_block = [&]() {
+        if (LIST && w < a.nworkers) nblock = __ldg(a.blocks + w * a.ppw / BLOCK_PASSES);
+    };
     auto draw = [&]() {
         if (!queue)
             w += gwarps;
         else if (lane == 0)
             w = gwarps + atomicAdd(a.ticket, 1);
+        find_block();
     };
+    find_block();
     // the pass after the one in the stage: the lane's row and its bounds, loaded one pass ahead
     int pass = 0, pass_end = 0, nrow = 0, nstart = 0, nend = 0;
     auto fetch_next = [&]() {
@@ -143,9 +155,10 @@ __global__ void __launch_bounds__(ROW_WARPS * 32, (row_min_ctas<P, NG>())) k_row
             }
             pass = t * a.ppw;
             pass_end = min(pass + a.ppw, a.npasses);
+            if constexpr (LIST) base = nblock - pass / BLOCK_PASSES * BATCH_BLOCK;
             draw();
         }
-        nrow = pass * R + lane / T;
+        nrow = base + pass * R + lane / T;
         nstart = __ldg(a.row_ptr + min(nrow, a.m));
         nend = __ldg(a.row_ptr + min(nrow + 1, a.m));
     };
@@ -275,6 +288,8 @@ __global__ void __launch_bounds__(ROW_WARPS * 32, (row_min_ctas<P, NG>())) k_row
         for (int d = 1; d < T; d <<= 1) acc = P::add(acc, sh_xor(acc, d));
         if (j == 0 && my_row < a.m) a.y[my_row] = P::out_acc(acc);
     }
+    if (LIST && blockIdx.x == 0 && threadIdx.x == 0)
+        asm volatile("griddepcontrol.wait;" ::: "memory");
     if (queue && lane == 0) {
         __threadfence();  // this warp's last draw comes before its count
         if (atomicAdd(a.ticket + 1, 1) == gwarps - 1) {  // every warp has drawn for the last time
@@ -284,10 +299,10 @@ __global__ void __launch_bounds__(ROW_WARPS * 32, (row_min_ctas<P, NG>())) k_row
     }
 }
 
-template <class P, int T, int NG>
+template <class P, int T, int NG, bool LIST = false>
 cudaError_t launch_row_kernel(const RowLaunch& l, cudaStream_t st) {
     constexpr int bytes = ROW_WARPS * RowStage<P, NG>::WARP_BYTES;
-    auto* const kernel = &k_rows<P, T, NG>;
+    auto* const kernel = &k_rows<P, T, NG, LIST>;
     // resident CTAs per SM; 0: the shared-memory opt-in is not set on this device yet (setting
     // it twice from racing host threads is harmless)
     static std::atomic<int> ctas_of[64];
@@ -314,14 +329,30 @@ cudaError_t launch_row_kernel(const RowLaunch& l, cudaStream_t st) {
     a.m = l.m;
     a.nnz = l.nnz;
     a.rotate = l.form.rotate;
-    a.npasses = (int)(((long long)l.m * T + 31) / 32);
+    a.blocks = l.blocks;
+    a.npasses = LIST ? l.nblocks * (BATCH_BLOCK * T / 32) : (int)(((long long)l.m * T + 31) / 32);
     const long long ctas = (long long)device_sm_count() * per_sm;
     const long long warps = ctas * ROW_WARPS;
     a.by_ticket = row_ticket_pays<P, NG>() && a.npasses >= 8 * warps;
     a.ppw = a.by_ticket ? 4 : a.npasses >= 4 * warps ? 2 : 1;
     a.nworkers = (a.npasses + a.ppw - 1) / a.ppw;
     const long long need = ((long long)a.nworkers + ROW_WARPS - 1) / ROW_WARPS;
-    kernel<<<(int)(need < ctas ? need : ctas), ROW_WARPS * 32, bytes, st>>>(a);
+    const int grid = (int)(need < ctas ? need : ctas);
+    if constexpr (LIST) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(grid);
+        cfg.blockDim = dim3(ROW_WARPS * 32);
+        cfg.dynamicSmemBytes = bytes;
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = l.dependent ? 1 : 0;
+        e = cudaLaunchKernelEx(&cfg, kernel, a);
+        return e != cudaSuccess ? e : cudaGetLastError();
+    }
+    kernel<<<grid, ROW_WARPS * 32, bytes, st>>>(a);
     return cudaGetLastError();
 }
 

@@ -1,16 +1,20 @@
 // spmv_batched.cu -- the batched multi-RHS form: many CSR matrices of uneven size, k in
 // {1, 2, 4, 8} right-hand sides, FP32 storage with the compensated FP32 arithmetic of the mixed
-// form, in one persistent launch replayed from a CUDA graph.  No counterpart in the reference.
+// form, replayed from a CUDA graph.  No counterpart in the reference.
 //
 // The batch is one block-diagonal CSR: the matrices' rows are concatenated (row_ptr carries
 // global non-zero offsets) and their column indices are offset into one concatenated x.  x and
 // y hold the k right-hand sides interleaved ([row][k]), so one gather brings all k values of an
-// x entry (k*4 bytes, one 256-bit load at k = 8).  One tile partition covers the whole batch;
-// the per-matrix tile counts are its segments.  A persistent kernel sized to the GPU's resident
-// capacity hands out workers (consecutive tile ranges) from a global atomic ticket, so the
-// uneven matrices load-balance over the SMs; the calibration kernel then adds the carry
-// records.  The persistent kernel and the calibration are captured once in a CUDA graph and
-// replayed by every call (the kernel leaves its ticket at zero for the next launch).
+// x entry (k*4 bytes, one 256-bit load at k = 8).
+//
+// A batch in which rows of whole-lane shape hold at least a quarter of the non-zeros runs over work
+// lists: row workers for the blocks of 256 rows that suit lanes on whole rows, tile workers for the
+// runs between them (batch_kernel.cuh; batch_k1.cu at one right-hand side).  Else, and where a
+// variant is forced, one tile partition covers the whole batch: a persistent kernel sized to the
+// GPU's resident capacity hands out workers (consecutive tile ranges) from a global atomic ticket,
+// so that the uneven matrices load-balance over the SMs, and the calibration kernel adds the carry
+// records.  Either way the kernels are captured once in a CUDA graph and replayed by every call
+// (tickets are left at zero for the next launch).
 #include <algorithm>
 #include <cstdio>
 #include <string>
@@ -169,6 +173,7 @@ static void batch_release(bhsp_batch* b) {
     cudaFree(b->ticket);
     cudaFree(b->work.tiles);
     cudaFree(b->work.rows);
+    cudaFree(b->work.blocks);
     cudaFree(b->work.tile_ptr);
     cudaFree(b->work.rec_row);
     cudaFree(b->work.rec_val);
@@ -196,20 +201,21 @@ static int batch_tiles_per_worker(const bhsp_batch* b) {
     return tpw;
 }
 
-// The batch's work lists (see batch_kernel.cuh), from two right-hand sides on: row workers for the
-// blocks of 256 rows that suit lanes on whole rows, tile workers for the runs between them.  Leaves
-// b->mixed false where the row workers would hold less than a quarter of the batch.
-//  * One right-hand side keeps the one tile kernel: on the 64-matrix mix the two kernels took 131
-//    against 137 us, on 128 matrices 238 against 232 us.
-//  * A block suits the row workers where its longest row fits (224 non-zeros) and its rows fill 0.4
-//    of the slots that their passes walk.  Random columns are no bar here: an x entry is 8 to 32
-//    bytes, its own sector or a good part of one, whichever lane reads it.  64 matrices of
-//    uniform density (Poisson rows of up to 20, random columns): 167 -> 128, 247 -> 158 and 280 ->
-//    216 us at 2, 4 and 8 right-hand sides; thresholds of 0.2 to 0.5 differ by 3 %.
+// The batch's work lists (see batch_kernel.cuh): row workers for the blocks of 256 rows that suit
+// lanes on whole rows, tile workers for the runs between them.  Leaves b->mixed false where the row
+// workers would hold less than a quarter of the batch.
+//  * A block suits the row workers where its longest row fits (224 non-zeros; 112 at one right-hand
+//    side) and its rows fill 0.4 of the slots that their passes walk.  Random columns are no bar
+//    here: an x entry is 8 to 32 bytes, its own sector or a good part of one, whichever lane reads
+//    it.  64 matrices of uniform density (Poisson rows of up to 20, random columns): 147 -> 107,
+//    167 -> 128, 247 -> 158 and 280 -> 216 us at 1, 2, 4 and 8 right-hand sides; thresholds of 0.2
+//    to 0.5 differ by 3 %.
+//  * One right-hand side runs one kernel per lane layout, so a layout with fewer passes than the
+//    GPU holds warps gives its blocks to the next larger one instead of a launch of its own.
 static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
     const int nblocks = (int)(((long long)b->m + BATCH_BLOCK - 1) / BATCH_BLOCK);
     // (row numbers of whole passes must not pass 2^31)
-    if (b->k == 1 || b->nnz == 0 || b->m > 0x7fffff00) return cudaSuccess;
+    if (b->nnz == 0 || b->m > 0x7fffff00) return cudaSuccess;
     std::vector<BlockStat> stat((size_t)nblocks);
     BlockStat* d_stat = nullptr;
     cudaError_t e = cudaMalloc(&d_stat, sizeof(BlockStat) * (size_t)nblocks);
@@ -226,10 +232,15 @@ static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
         const BlockStat& s = stat[(size_t)i];
         const int nnz = nnz_to(i + 1) - s.first;
         if (nnz == 0) return 0;
-        if (s.max_len > 8 * BATCH_SLOTS) return -1;
+        if (s.max_len > (b->k == 1 ? 4 : 8) * BATCH_SLOTS) return -1;
         int t = 0;
         while (s.max_len > BATCH_SLOTS << t) ++t;
         if (nnz < 0.4 * 128.0 * s.groups[t]) return -1;
+        if (b->k == 1) {  // the smallest layout of T lanes that holds the longest row
+            int f = 0;
+            while (LIST_FORMS[f].lanes < 1 << t || s.max_len > 4 * LIST_FORMS[f].groups << t) ++f;
+            return f;
+        }
         return t | (2 * s.eights > s.filled ? 8 : 0);
     };
     std::vector<int> form((size_t)nblocks);
@@ -246,7 +257,7 @@ static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
     // non-zeros were 0-5 % slower, on 5 and 16 matrices up to 38 %
     long long passes = 0;
     for (int i = 0; i < nblocks; ++i)
-        if (form[(size_t)i] >= 0) passes += BATCH_BLOCK / 32 << (form[(size_t)i] & 7);
+        if (b->k > 1 && form[(size_t)i] >= 0) passes += BATCH_BLOCK / 32 << (form[(size_t)i] & 7);
     const int ppw = (int)std::min<long long>(std::max<long long>(passes / (6 * warps), 1), 2);
     const int tpw = (int)std::min<long long>(
         {b->cfg.tiles_per_worker, std::max(1024 / tile, 1),
@@ -254,6 +265,8 @@ static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
     std::vector<RowWork> rows;
     std::vector<TileWork> tiles;
     std::vector<TileRun> runs;
+    std::vector<int> blocks[NLIST_FORMS];
+    int rotate[NLIST_FORMS] = {};  // blocks of a list whose rows start in the same banks
     int nbounds = 0;
     for (int i = 0; i < nblocks;) {
         const int f = form[(size_t)i];
@@ -261,7 +274,12 @@ static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
         while (j < nblocks && form[(size_t)j] == f) ++j;
         const int row0 = i * BATCH_BLOCK;
         const int row1 = (int)std::min<long long>((long long)j * BATCH_BLOCK, b->m);
-        if (f >= 0) {
+        if (f >= 0 && b->k == 1) {
+            for (int at = i; at < j; ++at) {
+                blocks[f].push_back(at * BATCH_BLOCK);
+                rotate[f] += 2 * stat[(size_t)at].eights > stat[(size_t)at].filled;
+            }
+        } else if (f >= 0) {
             const int step = std::max(ppw * (32 >> (f & 7)), 1);
             for (long long r = row0; r < row1; r += step)
                 rows.push_back(RowWork{f, (int)r, (int)std::min<long long>(r + step, row1)});
@@ -275,13 +293,32 @@ static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
         }
         i = j;
     }
-    for (int i = 0; i < (int)tiles.size(); i += 32)
-        rows.push_back(RowWork{-1, i, std::min(i + 32, (int)tiles.size())});
     BatchWork& w = b->work;
+    std::vector<int> listed;
+    for (int f = 0; f < NLIST_FORMS; ++f) {
+        const ListForm& form_f = LIST_FORMS[f];
+        if (blocks[f].empty()) continue;
+        const int up = form_f.into;
+        if (up >= 0 && (long long)blocks[f].size() * (BATCH_BLOCK / 32 * form_f.lanes) < warps) {
+            blocks[up].insert(blocks[up].end(), blocks[f].begin(), blocks[f].end());
+            rotate[up] += rotate[f];
+            continue;
+        }
+        RowList& l = w.lists[w.nlists++];
+        l.form.lanes = form_f.lanes;
+        l.form.groups = form_f.groups;
+        l.form.rotate = 2 * rotate[f] > (int)blocks[f].size();
+        l.first = (int)listed.size();
+        l.count = (int)blocks[f].size();
+        listed.insert(listed.end(), blocks[f].begin(), blocks[f].end());
+    }
+    for (int i = 0; b->k > 1 && i < (int)tiles.size(); i += 32)
+        rows.push_back(RowWork{-1, i, std::min(i + 32, (int)tiles.size())});
     w.ntiles = (int)tiles.size();
     w.nrows = (int)rows.size();
     TileRun* d_runs = nullptr;
-    e = cudaMalloc(&w.rows, sizeof(RowWork) * rows.size());
+    e = cudaMalloc(&w.rows, sizeof(RowWork) * (rows.size() + 1));
+    if (e == cudaSuccess) e = cudaMalloc(&w.blocks, sizeof(int) * (listed.size() + 1));
     if (e == cudaSuccess) e = cudaMalloc(&w.tiles, sizeof(TileWork) * (tiles.size() + 1));
     if (e == cudaSuccess) e = cudaMalloc(&w.tile_ptr, sizeof(uint32_t) * (size_t)(nbounds + 1));
     if (e == cudaSuccess) e = cudaMalloc(&w.rec_row, sizeof(int) * (tiles.size() + 1));
@@ -289,7 +326,10 @@ static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
     if (e == cudaSuccess) e = cudaMalloc(&w.row_ticket, 2 * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&d_runs, sizeof(TileRun) * (runs.size() + 1));
     if (e == cudaSuccess) e = cudaMemsetAsync(w.row_ticket, 0, 2 * sizeof(int), st);
-    if (e == cudaSuccess)
+    if (e == cudaSuccess && !listed.empty())
+        e = cudaMemcpyAsync(w.blocks, listed.data(), sizeof(int) * listed.size(),
+                            cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && !rows.empty())
         e = cudaMemcpyAsync(w.rows, rows.data(), sizeof(RowWork) * rows.size(),
                             cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && !tiles.empty())
@@ -304,6 +344,7 @@ static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
     cudaFree(d_runs);
     if (e != cudaSuccess) return e;
     switch (b->k) {
+        case 1: batch_work_grids<1>(b->cfg.seg, &w.tiles_grid, &w.rows_grid); break;
         case 2: batch_work_grids<2>(b->cfg.seg, &w.tiles_grid, &w.rows_grid); break;
         case 4: batch_work_grids<4>(b->cfg.seg, &w.tiles_grid, &w.rows_grid); break;
         default: batch_work_grids<8>(b->cfg.seg, &w.tiles_grid, &w.rows_grid); break;
@@ -418,6 +459,7 @@ static BatchLaunch batch_launch(bhsp_batch* b, const float* val, const void* x, 
 static cudaError_t enqueue(bhsp_batch* b, const BatchLaunch& l, cudaStream_t st) {
     if (!batch_takes_work(b)) return enqueue_batch(l, b->k, b->cfg, b->var, b->grid, st);
     switch (b->k) {
+        case 1: return launch_batch_work<1>(l, b->work, b->cfg.seg, st);
         case 2: return launch_batch_work<2>(l, b->work, b->cfg.seg, st);
         case 4: return launch_batch_work<4>(l, b->work, b->cfg.seg, st);
         default: return launch_batch_work<8>(l, b->work, b->cfg.seg, st);
@@ -437,7 +479,7 @@ extern "C" int bhsp_batch_execute(bhsp_batch* b, const float* d_val, const float
         return e == cudaSuccess ? BHSPARSE_SUCCESS : batch_cuda(b, e, "batched launch");
     }
     if (!b->exec || b->g_val != d_val || b->g_x != d_x || b->g_y != d_y) {
-        // (re)capture the persistent kernel and the calibration
+        // (re)capture the batch's kernels
         if (b->exec) cudaGraphExecDestroy(b->exec);
         if (b->graph) cudaGraphDestroy(b->graph);
         b->exec = nullptr;
@@ -487,7 +529,9 @@ extern "C" int bhsp_batch_info(const bhsp_batch* b, int* ntiles, int* nworkers, 
     if (nworkers) *nworkers = b->nworkers;
     if (grid) *grid = batch_takes_work(b) ? b->work.rows_grid : b->grid;
     if (launches)
-        *launches = batch_takes_work(b) ? (b->work.ntiles > 0 ? 2 : 1) : (b->nworkers > 0 ? 2 : 1);
+        *launches = !batch_takes_work(b) ? (b->nworkers > 0 ? 2 : 1)
+                    : b->k == 1          ? b->work.nlists + (b->work.ntiles > 0 ? 2 : 0)
+                                         : (b->work.ntiles > 0 ? 2 : 1);
     return BHSPARSE_SUCCESS;
 }
 

@@ -208,17 +208,17 @@ int bhsp_validate_csr(const int* d_row_ptr, const int* d_col_idx, int m, int n, 
  *   d_row_ptr[m_total+1]: the matrices' row pointers concatenated, with global non-zero offsets;
  *   d_col_idx[nnz_total]: each matrix's column indices plus the offset of its x block
  *                         (32-byte aligned).
- * x is [n_total][k] and y is [m_total][k], the k values of a row interleaved.  One persistent
- * kernel hands out tile ranges from a global ticket; schedule fields as in bhsp_set_config
- * (0 = default: seg 16, or 32 for k = 4; 1 to 4 tiles per worker by the batch's size; 4 warps
- * per CTA).  Validates the
- * CSR and builds the partition (synchronous). */
+ * x is [n_total][k] and y is [m_total][k], the k values of a row interleaved.  Blocks of short,
+ * even rows run with lanes on whole rows, the others by tile ranges drawn from a global ticket;
+ * schedule fields, for the latter, as in bhsp_set_config (0 = default: seg 16, or 32 for k = 4;
+ * 1 to 4 tiles per worker by the batch's size; 4 warps per CTA).  Validates the CSR and builds the
+ * partition (synchronous). */
 typedef struct bhsp_batch bhsp_batch;
 int bhsp_batch_create(bhsp_batch** out, int count, int m_total, int n_total, int nnz_total,
                       const int* d_row_ptr, const int* d_col_idx, int k, int seg,
                       int tiles_per_worker, int warps_per_cta, void* stream);
 /* y = A.x for all matrices and right-hand sides, enqueued on `stream`.  use_graph != 0 replays a
- * CUDA graph of the persistent kernel and the calibration (captured on the
+ * CUDA graph of the batch's kernels (captured on the
  * first call and again whenever the buffers change); use_graph == 0 launches them directly.
  * d_val 32-byte aligned, d_x / d_y aligned to 4*k bytes. */
 int bhsp_batch_execute(bhsp_batch* b, const float* d_val, const float* d_x, float* d_y,
