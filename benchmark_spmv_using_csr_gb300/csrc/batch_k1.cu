@@ -3,8 +3,8 @@
 // Tile workers as at 2 to 8 right-hand sides; the row blocks, by the lane layout that suits them, in
 // one launch of the row kernel (row_kernel.cuh) per layout, each the programmatic dependent of the
 // one before: it starts as that one drains, which hides the tails.  A layout known at compile time is
-// what makes the difference: with a run-time one, as k_batch_rows has it, a non-zero takes about 20
-// instructions, as many as the tile kernel (64 matrices: 131 us).
+// what makes the difference: with a run-time one a non-zero takes about 20 instructions, as many as
+// the tile kernel (64 matrices: 131 us).
 //
 // Bound by memory in the regular members (27-point stencils 6830 GB/s, 32 x 32 blocks 6650) and by
 // latency in the tile workers'.  Measured against the tile kernel over the whole batch: 128 matrices of
@@ -32,41 +32,22 @@ cudaError_t launch_rows_listed(const RowLaunch& l, cudaStream_t st) {
 }
 
 // the tile workers' carry records, once every kernel before is done
-__global__ void k_batch_calibrate(BatchArgs<1> a) {
+__global__ void k_batch_calibrate(const int* rec_row, const VecD<1>* rec_val, int nrec, VecF<1>* y,
+                                  int m, uint32_t* err) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int warp = (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5));
     const int warps = (int)(gridDim.x * (blockDim.x >> 5));
-    for (int base = warp * 32; base < a.nrec; base += warps * 32)
-        calibrate_records<PolMixedK<1>>(a.t.rec_row, a.t.rec_val, a.nrec, base, a.t.y, a.t.m, a.t.err);
+    for (int base = warp * 32; base < nrec; base += warps * 32)
+        calibrate_records<PolMixedK<1>>(rec_row, rec_val, nrec, base, y, m, err);
 }
 
-template <>
-void batch_work_grids<1>(int seg, int* tiles, int* rows) {
-    *tiles = seg == 8    ? batch_tiles_grid<1, 8>()
-             : seg == 16 ? batch_tiles_grid<1, 16>()
-                         : batch_tiles_grid<1, 32>();
-    *rows = *tiles;
-}
+template int batch_work_grid<1>(int);
 
 template <>
 cudaError_t launch_batch_work<1>(const BatchLaunch& l, const BatchWork& b, int seg,
                                  cudaStream_t st) {
-    BatchArgs<1> a;
-    a.t = batch_tile_args<1>(l);
-    a.t.tile_ptr = b.tile_ptr;
-    a.t.rec_row = b.rec_row;
-    a.t.rec_val = static_cast<VecD<1>*>(b.rec_val);
-    a.tiles = b.tiles;
-    a.rows = nullptr;
-    a.ntiles = a.nrec = b.ntiles;
-    a.nrows = 0;
-    a.row_ticket = nullptr;
-    if (b.ntiles > 0) {
-        auto* const kernel = seg == 8    ? batch_tiles_kernel<1, 8>()
-                             : seg == 16 ? batch_tiles_kernel<1, 16>()
-                                         : batch_tiles_kernel<1, 32>();
-        kernel<<<b.tiles_grid, BATCH_WARPS * 32, 0, st>>>(a);
-    }
+    cudaError_t e = launch_batch_tiles<1>(l, b, seg, st);
+    if (e != cudaSuccess) return e;
     RowLaunch r;
     r.row_ptr = l.row_ptr;
     r.col = l.col;
@@ -82,7 +63,7 @@ cudaError_t launch_batch_work<1>(const BatchLaunch& l, const BatchWork& b, int s
         r.blocks = b.blocks + b.lists[i].first;
         r.nblocks = b.lists[i].count;
         r.dependent = i > 0 || b.ntiles > 0;
-        const cudaError_t e = launch_rows_listed(r, st);
+        e = launch_rows_listed(r, st);
         if (e != cudaSuccess) return e;
     }
     if (b.ntiles > 0) {
@@ -95,7 +76,9 @@ cudaError_t launch_batch_work<1>(const BatchLaunch& l, const BatchWork& b, int s
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, k_batch_calibrate, a);
+        e = cudaLaunchKernelEx(&cfg, k_batch_calibrate, b.rec_row,
+                               static_cast<const VecD<1>*>(b.rec_val), b.ntiles,
+                               static_cast<VecF<1>*>(l.y), l.m, l.err);
         if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();

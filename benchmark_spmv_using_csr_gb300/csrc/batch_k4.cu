@@ -3,7 +3,7 @@
 
 namespace spmv {
 
-template void batch_work_grids<4>(int, int*, int*);
+template int batch_work_grid<4>(int);
 template cudaError_t launch_batch_work<4>(const BatchLaunch&, const BatchWork&, int, cudaStream_t);
 
 }  // namespace spmv

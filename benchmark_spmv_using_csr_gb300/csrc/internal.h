@@ -160,41 +160,36 @@ struct BatchLaunch {
     int* ticket;
     int m, n, nnz;
 };
-// A row worker: rows [first, last) with 1 << (form & 7) lanes per row (bit 3: rotated slots); or,
-// form < 0, the carry records [first, last) of the tile workers to add to their rows.
-struct RowWork {
-    int form, first, last;
-};
 // A tile worker: tiles [first, last) of the run of rows [row0, row1), its part of tile_ptr (tile t's
 // entry is tile_ptr[at + t]); its carry record has the worker's number.
 struct TileWork {
     int first, last, row0, row1, at;
 };
 constexpr int BATCH_SLOTS = 28;  // of a lane in a pass: rows of up to 28, 56, 112, 224 non-zeros
-// One right-hand side: the blocks whose rows one lane layout of the row kernel takes.
+// The blocks whose rows one lane layout takes.
 struct RowList {
     RowForm form;
     int first, count;  // blocks[first ...]
 };
-// lane layouts of the row lists, smaller ones first: lanes per row, groups of 4 slots per lane, and
-// the layout that takes its blocks too where they are too few for a kernel of their own (-1: none)
+// Lane layouts of the row lists, smaller ones first: lanes per row, groups of 4 slots per lane, and
+// the layout that takes its blocks too where they are too few for a kernel of their own (-1: none).
 struct ListForm {
     int lanes, groups, into;
 };
-constexpr ListForm LIST_FORMS[] = {{1, 2, 1}, {1, 4, 2}, {1, 7, -1}, {2, 4, 4}, {2, 7, -1}, {4, 7, -1}};
-constexpr int NLIST_FORMS = sizeof(LIST_FORMS) / sizeof(LIST_FORMS[0]);
+constexpr int NLIST_FORMS = 6;
+// at one right-hand side (batch_k1.cu; the groups are registers) and at 2, 4 and 8 (batch_kernel.cuh)
+constexpr ListForm LIST_FORMS_1[NLIST_FORMS] = {{1, 2, 1}, {1, 4, 2}, {1, 7, 3},
+                                                {2, 4, 4}, {2, 7, 5}, {4, 7, -1}};
+constexpr ListForm LIST_FORMS_K[NLIST_FORMS] = {{1, 3, 1}, {1, 7, 2}, {2, 7, 3}, {4, 7, 4}, {8, 7, -1}};
 // The two work lists and their kernels' buffers.
 struct BatchWork {
     TileWork* tiles = nullptr;  // [ntiles]
-    RowWork* rows = nullptr;    // [nrows], the carry records' workers last
-    int* blocks = nullptr;      // one right-hand side: first rows of blocks, list by list
+    int* blocks = nullptr;      // first rows of the row blocks, list by list
     RowList lists[NLIST_FORMS];
-    int nlists = 0;
     uint32_t* tile_ptr = nullptr;
-    int* rec_row = nullptr;     // [ntiles]
+    int* rec_row = nullptr;  // [ntiles]
     void* rec_val = nullptr;
-    int* row_ticket = nullptr;  // [2], as the tile kernel's
-    int ntiles = 0, nrows = 0, tiles_grid = 0, rows_grid = 0;
+    int ntiles = 0, nlists = 0, tiles_grid = 0;
 };
 // What the work lists need of each block of 256 rows.
 struct BlockStat {

@@ -335,11 +335,9 @@ TileArgs<PolMixedK<K>> batch_tile_args(const BatchLaunch& l) {
 
 // batch_k<K>.cu
 template <int K>
-void batch_work_grids(int seg, int* tiles, int* rows);
+int batch_work_grid(int seg);
 template <int K>
 cudaError_t launch_batch_work(const BatchLaunch& l, const BatchWork& b, int seg, cudaStream_t st);
-template <>
-void batch_work_grids<1>(int seg, int* tiles, int* rows);
 template <>
 cudaError_t launch_batch_work<1>(const BatchLaunch& l, const BatchWork& b, int seg, cudaStream_t st);
 

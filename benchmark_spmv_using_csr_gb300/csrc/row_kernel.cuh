@@ -299,25 +299,32 @@ __global__ void __launch_bounds__(ROW_WARPS * 32, (row_min_ctas<P, NG>())) k_row
     }
 }
 
-template <class P, int T, int NG, bool LIST = false>
-cudaError_t launch_row_kernel(const RowLaunch& l, cudaStream_t st) {
-    constexpr int bytes = ROW_WARPS * RowStage<P, NG>::WARP_BYTES;
-    auto* const kernel = &k_rows<P, T, NG, LIST>;
-    // resident CTAs per SM; 0: the shared-memory opt-in is not set on this device yet (setting
-    // it twice from racing host threads is harmless)
-    static std::atomic<int> ctas_of[64];
+// A kernel's resident CTAs per SM on the current device, looked up once per device, with its
+// shared-memory opt-in (setting it twice from racing host threads is harmless).
+template <auto KERNEL>
+cudaError_t resident_ctas(int threads, int bytes, int* per_sm) {
+    static std::atomic<int> ctas_of[64];  // 0: not looked up
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    int per_sm = dev < 64 ? ctas_of[dev].load(std::memory_order_acquire) : 0;
-    if (per_sm == 0) {
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-        if (e == cudaSuccess)
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, ROW_WARPS * 32, bytes);
-        if (e != cudaSuccess) return e;
-        if (per_sm < 1) return cudaErrorInvalidConfiguration;
-        if (dev < 64) ctas_of[dev].store(per_sm, std::memory_order_release);
-    }
+    *per_sm = dev < 64 ? ctas_of[dev].load(std::memory_order_acquire) : 0;
+    if (*per_sm > 0) return cudaSuccess;
+    e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, KERNEL, threads, bytes);
+    if (e != cudaSuccess) return e;
+    if (*per_sm < 1) return cudaErrorInvalidConfiguration;
+    if (dev < 64) ctas_of[dev].store(*per_sm, std::memory_order_release);
+    return cudaSuccess;
+}
+
+template <class P, int T, int NG, bool LIST = false>
+cudaError_t launch_row_kernel(const RowLaunch& l, cudaStream_t st) {
+    constexpr int bytes = ROW_WARPS * RowStage<P, NG>::WARP_BYTES;
+    constexpr auto kernel = &k_rows<P, T, NG, LIST>;
+    int per_sm = 0;
+    cudaError_t e = resident_ctas<kernel>(ROW_WARPS * 32, bytes, &per_sm);
+    if (e != cudaSuccess) return e;
     RowArgs<P> a;
     a.row_ptr = l.row_ptr;
     a.col = l.col;

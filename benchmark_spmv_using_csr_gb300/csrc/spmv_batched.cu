@@ -172,12 +172,10 @@ static void batch_release(bhsp_batch* b) {
     cudaFree(b->err);
     cudaFree(b->ticket);
     cudaFree(b->work.tiles);
-    cudaFree(b->work.rows);
     cudaFree(b->work.blocks);
     cudaFree(b->work.tile_ptr);
     cudaFree(b->work.rec_row);
     cudaFree(b->work.rec_val);
-    cudaFree(b->work.row_ticket);
     b->work = BatchWork{};
     b->exec = nullptr;
     b->graph = nullptr;
@@ -210,8 +208,13 @@ static int batch_tiles_per_worker(const bhsp_batch* b) {
 //    it.  64 matrices of uniform density (Poisson rows of up to 20, random columns): 147 -> 107,
 //    167 -> 128, 247 -> 158 and 280 -> 216 us at 1, 2, 4 and 8 right-hand sides; thresholds of 0.2
 //    to 0.5 differ by 3 %.
-//  * One right-hand side runs one kernel per lane layout, so a layout with fewer passes than the
-//    GPU holds warps gives its blocks to the next larger one instead of a launch of its own.
+//  * Each lane layout is a kernel of its own, so one with fewer passes than the GPU holds warps gives
+//    its blocks to the next larger one, the last one to the tile workers.  (Half and twice that
+//    bound differ by up to 10 % either way on 8 and 16 matrices; two blocks of the last layout as a
+//    kernel of their own took 15-25 us of a 64-matrix batch.)
+//  * From two right-hand sides on the layouts of many lanes run first: their passes are the longest.
+//    64 matrices 127.5, 161 and 236 -> 119.5, 149 and 230 us at 2, 4 and 8; at one right-hand side 64
+//    matrices 110 -> 108, but 8 and 16 matrices 27 -> 31 and 51 -> 54, so there they run last.
 static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
     const int nblocks = (int)(((long long)b->m + BATCH_BLOCK - 1) / BATCH_BLOCK);
     // (row numbers of whole passes must not pass 2^31)
@@ -226,8 +229,11 @@ static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     cudaFree(d_stat);
     if (e != cudaSuccess) return e;
+    const int tile = 32 * b->cfg.seg;
+    const long long warps = (long long)device_sm_count() * 16;
     auto nnz_to = [&](int i) { return i < nblocks ? stat[(size_t)i].first : b->nnz; };
-    // the row form of a block, or -1
+    const ListForm* const forms = b->k == 1 ? LIST_FORMS_1 : LIST_FORMS_K;
+    // the layout of a block, or -1
     auto form_of = [&](int i) -> int {
         const BlockStat& s = stat[(size_t)i];
         const int nnz = nnz_to(i + 1) - s.first;
@@ -236,33 +242,35 @@ static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
         int t = 0;
         while (s.max_len > BATCH_SLOTS << t) ++t;
         if (nnz < 0.4 * 128.0 * s.groups[t]) return -1;
-        if (b->k == 1) {  // the smallest layout of T lanes that holds the longest row
-            int f = 0;
-            while (LIST_FORMS[f].lanes < 1 << t || s.max_len > 4 * LIST_FORMS[f].groups << t) ++f;
-            return f;
-        }
-        return t | (2 * s.eights > s.filled ? 8 : 0);
+        int f = 0;  // the smallest layout of T lanes that holds the longest row
+        while (forms[f].lanes < 1 << t || s.max_len > 4 * forms[f].groups << t) ++f;
+        return f;
     };
     std::vector<int> form((size_t)nblocks);
+    long long count[NLIST_FORMS] = {};  // blocks by layout
+    for (int i = 0; i < nblocks; ++i)
+        if ((form[(size_t)i] = form_of(i)) >= 0) ++count[form[(size_t)i]];
+    // the layout that takes a layout's blocks (-1: the tile workers)
+    int taken[NLIST_FORMS];
+    for (int f = 0; f < NLIST_FORMS; ++f) {
+        const long long passes = count[f] * (BATCH_BLOCK / 32) * forms[f].lanes;
+        const int up = forms[f].into;
+        const bool few = up >= 0 ? passes < warps : 4 * passes < warps;
+        taken[f] = few ? up : f;
+        if (few && up >= 0) count[up] += count[f];
+    }
     long long row_nnz = 0;
     for (int i = 0; i < nblocks; ++i) {
-        form[(size_t)i] = form_of(i);
-        if (form[(size_t)i] >= 0) row_nnz += nnz_to(i + 1) - stat[(size_t)i].first;
+        int& f = form[(size_t)i];
+        while (f >= 0 && taken[f] != f) f = taken[f];
+        if (f >= 0) row_nnz += nnz_to(i + 1) - stat[(size_t)i].first;
     }
     if (4 * row_nnz < b->nnz) return cudaSuccess;
-    const int tile = 32 * b->cfg.seg;
-    const long long warps = (long long)device_sm_count() * 16;
-    // passes per row worker (up to 2) and tiles per tile worker (up to 1024 non-zeros), as many as
-    // leave every warp several workers: on the 64-matrix mix 4 and 8 passes or 2048 and 4096
-    // non-zeros were 0-5 % slower, on 5 and 16 matrices up to 38 %
-    long long passes = 0;
-    for (int i = 0; i < nblocks; ++i)
-        if (b->k > 1 && form[(size_t)i] >= 0) passes += BATCH_BLOCK / 32 << (form[(size_t)i] & 7);
-    const int ppw = (int)std::min<long long>(std::max<long long>(passes / (6 * warps), 1), 2);
+    // tiles per tile worker (up to 1024 non-zeros), as many as leave every warp several workers: on
+    // the 64-matrix mix 2048 and 4096 non-zeros were 0-5 % slower, on 5 and 16 matrices up to 38 %
     const int tpw = (int)std::min<long long>(
         {b->cfg.tiles_per_worker, std::max(1024 / tile, 1),
          (int)std::max<long long>((b->nnz - row_nnz) / tile / (6 * warps), 1)});
-    std::vector<RowWork> rows;
     std::vector<TileWork> tiles;
     std::vector<TileRun> runs;
     std::vector<int> blocks[NLIST_FORMS];
@@ -274,15 +282,11 @@ static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
         while (j < nblocks && form[(size_t)j] == f) ++j;
         const int row0 = i * BATCH_BLOCK;
         const int row1 = (int)std::min<long long>((long long)j * BATCH_BLOCK, b->m);
-        if (f >= 0 && b->k == 1) {
+        if (f >= 0) {
             for (int at = i; at < j; ++at) {
                 blocks[f].push_back(at * BATCH_BLOCK);
                 rotate[f] += 2 * stat[(size_t)at].eights > stat[(size_t)at].filled;
             }
-        } else if (f >= 0) {
-            const int step = std::max(ppw * (32 >> (f & 7)), 1);
-            for (long long r = row0; r < row1; r += step)
-                rows.push_back(RowWork{f, (int)r, (int)std::min<long long>(r + step, row1)});
         } else {
             TileRun r{row0, row1, nnz_to(i) / tile, (int)(((long long)nnz_to(j) + tile - 1) / tile),
                       nbounds};
@@ -295,42 +299,27 @@ static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
     }
     BatchWork& w = b->work;
     std::vector<int> listed;
-    for (int f = 0; f < NLIST_FORMS; ++f) {
-        const ListForm& form_f = LIST_FORMS[f];
+    for (int i = 0; i < NLIST_FORMS; ++i) {
+        const int f = b->k == 1 ? i : NLIST_FORMS - 1 - i;
         if (blocks[f].empty()) continue;
-        const int up = form_f.into;
-        if (up >= 0 && (long long)blocks[f].size() * (BATCH_BLOCK / 32 * form_f.lanes) < warps) {
-            blocks[up].insert(blocks[up].end(), blocks[f].begin(), blocks[f].end());
-            rotate[up] += rotate[f];
-            continue;
-        }
         RowList& l = w.lists[w.nlists++];
-        l.form.lanes = form_f.lanes;
-        l.form.groups = form_f.groups;
+        l.form.lanes = forms[f].lanes;
+        l.form.groups = forms[f].groups;
         l.form.rotate = 2 * rotate[f] > (int)blocks[f].size();
         l.first = (int)listed.size();
         l.count = (int)blocks[f].size();
         listed.insert(listed.end(), blocks[f].begin(), blocks[f].end());
     }
-    for (int i = 0; b->k > 1 && i < (int)tiles.size(); i += 32)
-        rows.push_back(RowWork{-1, i, std::min(i + 32, (int)tiles.size())});
     w.ntiles = (int)tiles.size();
-    w.nrows = (int)rows.size();
     TileRun* d_runs = nullptr;
-    e = cudaMalloc(&w.rows, sizeof(RowWork) * (rows.size() + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&w.blocks, sizeof(int) * (listed.size() + 1));
+    e = cudaMalloc(&w.blocks, sizeof(int) * (listed.size() + 1));
     if (e == cudaSuccess) e = cudaMalloc(&w.tiles, sizeof(TileWork) * (tiles.size() + 1));
     if (e == cudaSuccess) e = cudaMalloc(&w.tile_ptr, sizeof(uint32_t) * (size_t)(nbounds + 1));
     if (e == cudaSuccess) e = cudaMalloc(&w.rec_row, sizeof(int) * (tiles.size() + 1));
     if (e == cudaSuccess) e = cudaMalloc(&w.rec_val, sizeof(double) * b->k * (tiles.size() + 1));
-    if (e == cudaSuccess) e = cudaMalloc(&w.row_ticket, 2 * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&d_runs, sizeof(TileRun) * (runs.size() + 1));
-    if (e == cudaSuccess) e = cudaMemsetAsync(w.row_ticket, 0, 2 * sizeof(int), st);
     if (e == cudaSuccess && !listed.empty())
         e = cudaMemcpyAsync(w.blocks, listed.data(), sizeof(int) * listed.size(),
-                            cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && !rows.empty())
-        e = cudaMemcpyAsync(w.rows, rows.data(), sizeof(RowWork) * rows.size(),
                             cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && !tiles.empty())
         e = cudaMemcpyAsync(w.tiles, tiles.data(), sizeof(TileWork) * tiles.size(),
@@ -344,12 +333,12 @@ static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
     cudaFree(d_runs);
     if (e != cudaSuccess) return e;
     switch (b->k) {
-        case 1: batch_work_grids<1>(b->cfg.seg, &w.tiles_grid, &w.rows_grid); break;
-        case 2: batch_work_grids<2>(b->cfg.seg, &w.tiles_grid, &w.rows_grid); break;
-        case 4: batch_work_grids<4>(b->cfg.seg, &w.tiles_grid, &w.rows_grid); break;
-        default: batch_work_grids<8>(b->cfg.seg, &w.tiles_grid, &w.rows_grid); break;
+        case 1: w.tiles_grid = batch_work_grid<1>(b->cfg.seg); break;
+        case 2: w.tiles_grid = batch_work_grid<2>(b->cfg.seg); break;
+        case 4: w.tiles_grid = batch_work_grid<4>(b->cfg.seg); break;
+        default: w.tiles_grid = batch_work_grid<8>(b->cfg.seg); break;
     }
-    b->mixed = w.tiles_grid > 0 && w.rows_grid > 0;
+    b->mixed = w.tiles_grid > 0 && w.nlists > 0;
     return cudaSuccess;
 }
 
@@ -527,11 +516,11 @@ extern "C" int bhsp_batch_info(const bhsp_batch* b, int* ntiles, int* nworkers, 
     if (!b) return BHSPARSE_INVALID_ARGUMENT;
     if (ntiles) *ntiles = b->ntiles;
     if (nworkers) *nworkers = b->nworkers;
-    if (grid) *grid = batch_takes_work(b) ? b->work.rows_grid : b->grid;
+    if (grid) *grid = batch_takes_work(b) ? b->work.tiles_grid : b->grid;
     if (launches)
         *launches = !batch_takes_work(b) ? (b->nworkers > 0 ? 2 : 1)
-                    : b->k == 1          ? b->work.nlists + (b->work.ntiles > 0 ? 2 : 0)
-                                         : (b->work.ntiles > 0 ? 2 : 1);
+                    // (at one right-hand side the carry records are a kernel of their own)
+                    : b->work.nlists + (b->work.ntiles == 0 ? 0 : b->k == 1 ? 2 : 1);
     return BHSPARSE_SUCCESS;
 }
 
