@@ -377,9 +377,13 @@ cudaError_t launch_rows(const RowLaunch& l, cudaStream_t st) {
     SPMV_ROW_FORM(T, 6);   \
     SPMV_ROW_FORM(T, 7)
     SPMV_ROW_FORMS(1);
-    SPMV_ROW_FORMS(2);
-    SPMV_ROW_FORMS(4);
-    SPMV_ROW_FORMS(8);
+    if constexpr (sizeof(typename P::VS) == 8) {
+        SPMV_ROW_FORM(2, 4);  // FP64 rows have at most 32 non-zeros (choose_row_form)
+    } else {
+        SPMV_ROW_FORMS(2);
+        SPMV_ROW_FORMS(4);
+        SPMV_ROW_FORMS(8);
+    }
 #undef SPMV_ROW_FORMS
 #undef SPMV_ROW_FORM
     return cudaErrorInvalidValue;
