@@ -26,7 +26,7 @@
 //    registers; a matrix larger than one wave of workers runs a persistent kernel whose warps
 //    take workers from a global ticket, a smaller one a warp per worker.  The row it starts inside of (the reference's synchronizer entry,
 //    kernels_cuda.h:243-247) is the only value it cannot write itself; it goes to a
-//    per-worker carry record that k_calibrate adds in worker order after the main kernel
+//    per-worker carry record that k_calibrate adds in a fixed order after the main kernel
 //    (replacing the host loop of bhsparse_spmv_cuda.h:170-173).  Every other row is
 //    written exactly once, by the worker in which it starts, so y needs no zeroing and
 //    repeated calls give the same y.

@@ -157,7 +157,8 @@ int bhsp_plan_execute_phase(bhsp_plan* p, const void* d_val, const void* d_x, vo
                             void* stream, int phase);
 /* Synchronise `stream` and report (then clear) any kernel-side check that fired. */
 int bhsp_plan_check(bhsp_plan* p, void* stream);
-/* Number of device kernels one bhsp_plan_execute launches. */
+/* Number of device kernels one bhsp_plan_execute launches: 2, or 1 where the plan runs the row
+ * kernel (short, even rows: lanes on whole rows) or has no non-zeros. */
 int bhsp_plan_launches(const bhsp_plan* p);
 /* tile_ptr of the plan (device pointer, ntiles+1 entries) and its tile size. */
 int bhsp_plan_tiles(const bhsp_plan* p, const uint32_t** d_tile_ptr, int* ntiles, int* tile_nnz);
@@ -172,7 +173,8 @@ int bhsp_plan_chunk_form(const bhsp_plan* p, int* short_rows, int* one_head);
 int bhsp_plan_gather_path(const bhsp_plan* p, int* sampled, int* near, int* l2_only);
 /* Overrides the kernel variant the plan's rules chose: one_head (the chunk form above) and
  * l2_only (the gather path) = 1 or 0 to force it, -1 to keep the rule's choice.  Every variant
- * gives the same y; only the speed differs.  Takes effect at the next bhsp_plan_execute. */
+ * gives the same y; only the speed differs.  Takes effect at the next bhsp_plan_execute.  A plan
+ * with a forced variant or grid runs the tile kernel, whatever its rows. */
 int bhsp_plan_set_variant(bhsp_plan* p, int one_head, int l2_only);
 /* Overrides the grid of the direct-load tile kernel: 1 = the persistent kernel (warps draw
  * workers from the plan's work queue), 0 = a static grid of one warp per worker, -1 = the rule
@@ -224,6 +226,8 @@ int bhsp_batch_create(bhsp_batch** out, int count, int m_total, int n_total, int
 int bhsp_batch_execute(bhsp_batch* b, const float* d_val, const float* d_x, float* d_y,
                        int use_graph, void* stream);
 int bhsp_batch_check(bhsp_batch* b, void* stream);
+/* Tiles and workers of the partition over the whole batch, the grid of the tile workers' kernel
+ * and the device kernels of one execute. */
 int bhsp_batch_info(const bhsp_batch* b, int* ntiles, int* nworkers, int* grid, int* launches);
 /* The kernel variant bhsp_batch_create chose for the batch, as bhsp_plan_chunk_form /
  * bhsp_plan_gather_path do for one matrix: *one_head = 1 for the branch-free one-head chunk form
@@ -232,7 +236,8 @@ int bhsp_batch_info(const bhsp_batch* b, int* ntiles, int* nworkers, int* grid, 
 int bhsp_batch_variant(const bhsp_batch* b, int* one_head, int* l2_only);
 /* Overrides that choice: one_head / l2_only = 1 or 0 to force, -1 to keep.  The one-head form
  * exists for one right-hand side only (one_head = 1 with k > 1 is rejected).  Every variant
- * gives the same y; the next bhsp_batch_execute with use_graph captures the graph again. */
+ * gives the same y; the next bhsp_batch_execute with use_graph captures the graph again.  A batch
+ * with a forced variant runs the tile kernel over all its rows. */
 int bhsp_batch_set_variant(bhsp_batch* b, int one_head, int l2_only);
 /* The batched form's schedule tuner.  Candidates: S 8 / 16 / 32 x 1 / 2 / 4 / 8 tiles per
  * worker x 4 / 8 warps per CTA.  bhsp_batch_autotune builds the batch at every candidate and
