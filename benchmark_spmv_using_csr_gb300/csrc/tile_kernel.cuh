@@ -790,7 +790,7 @@ __device__ __forceinline__ void calibrate_records(const int* __restrict__ rec_ro
     const int re = (lane == 0 || lane == 31) && edge >= 0 && edge < nworkers ? rec_row[edge] : -1;
     const Rec none = P::rec_of_y(YT(0));
     Rec acc = none;
-    if (r >= 0) acc = rec_val[w];
+    if (w < nworkers) acc = rec_val[w];  // not used where the worker left no record (r < 0)
     int rprev = __shfl_up_sync(SPMV_FULL_MASK, r, 1);
     int rnext = __shfl_down_sync(SPMV_FULL_MASK, r, 1);
     if (lane == 0) rprev = re;
