@@ -809,7 +809,7 @@ def measure_batched(args) -> dict:
     out = {"matrices": len(mats), "nnz": nnz, "rows": sum(a.m for a in mats),
            "plain_fp64_sequential": {"ms_per_rhs": round(ms_plain, 4),
                                      "gnnz_per_s": round(nnz / ms_plain / 1e6, 2),
-                                     "launches_per_rhs": 2 * len(mats)}}
+                                     "launches_per_rhs": sum(p[0].launches for p in plans)}}
     for p in plans:
         p[0].close()
     del plans
