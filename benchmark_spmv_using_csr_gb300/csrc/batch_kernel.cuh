@@ -94,7 +94,8 @@ constexpr auto batch_tiles_kernel() {
 // A lane has U slots' x entries in flight while it multiplies the U before them.  U and the CTAs per
 // SM trade loads in flight against warps: on the 64-matrix mix K = 2 takes 120 us at U = 8 and 5 or
 // 6 CTAs, 130-140 at 4 or 7 CTAs or U of 4 or 6; K = 4 148 us at U = 4 and 5 or 6 CTAs, 160-168 at U of
-// 2 or 8; K = 8 229 us at U = 2 and 5 or 6 CTAs, 236 at U = 4 and 4.  Rows of up to 12 non-zeros have two stages per warp, since their passes are too
+// 2 or 8; K = 8 229 us at U = 2 and 5 or 6 CTAs, 236 at U = 4 and 4 (which is 6 % faster on 27-point
+// stencils and 32 x 32 blocks alone; for those layouts only it makes the mix 243).  Rows of up to 12 non-zeros have two stages per warp, since their passes are too
 // short to hide the next one's copies; longer ones one, since a second one of that size costs more in
 // L1 and warps than it hides (K = 2: 150 against 140 us).
 template <int K>

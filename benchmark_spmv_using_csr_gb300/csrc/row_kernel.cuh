@@ -11,7 +11,8 @@
 // Why lanes take rows here and consecutive non-zeros in tile_kernel.cuh: in a stencil or block
 // matrix neighbouring rows reference neighbouring columns, so that at slot k the 32 lanes read
 // a few consecutive runs of x (2-3 lines instead of about 10), and there are no bit flags, row
-// maps and segmented scans to pay for: about 12 instructions per non-zero and lane instead of 32.
+// maps and segmented scans to pay for: about 12 instructions per non-zero and lane instead of 32
+// in the plain forms.
 //
 // Measured on the 27-point stencil on 160^3 (109 M non-zeros), tile kernel at its best schedule
 // -> this one: mixed FP32 176 -> 136 us (6800 GB/s: memory-bound), FP64 262 -> 229 us (6090 GB/s;
