@@ -17,6 +17,7 @@
 // (tickets are left at zero for the next launch).
 #include <algorithm>
 #include <cstdio>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -163,6 +164,16 @@ struct bhsp_batch {
     std::string last_error;
 };
 
+static void batch_work_release(bhsp_batch* b) {
+    cudaFree(b->work.tiles);
+    cudaFree(b->work.blocks);
+    cudaFree(b->work.tile_ptr);
+    cudaFree(b->work.rec_row);
+    cudaFree(b->work.rec_val);
+    b->work = BatchWork{};
+    b->mixed = false;
+}
+
 static void batch_release(bhsp_batch* b) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
@@ -171,12 +182,7 @@ static void batch_release(bhsp_batch* b) {
     cudaFree(b->rec_val);
     cudaFree(b->err);
     cudaFree(b->ticket);
-    cudaFree(b->work.tiles);
-    cudaFree(b->work.blocks);
-    cudaFree(b->work.tile_ptr);
-    cudaFree(b->work.rec_row);
-    cudaFree(b->work.rec_val);
-    b->work = BatchWork{};
+    batch_work_release(b);
     b->exec = nullptr;
     b->graph = nullptr;
 }
@@ -342,6 +348,20 @@ static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
     return cudaSuccess;
 }
 
+// The work lists, or none where there is no memory for them: the one tile kernel needs none.
+static cudaError_t batch_work_try(bhsp_batch* b, cudaStream_t st) {
+    cudaError_t e = cudaSuccess;
+    try {
+        e = batch_work_build(b, st);
+    } catch (const std::bad_alloc&) {
+        e = cudaErrorMemoryAllocation;
+    }
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();  // clear the allocation's error
+    batch_work_release(b);
+    return cudaSuccess;
+}
+
 // Whether an execute runs the work list (else the tile kernel over the whole batch).
 static bool batch_takes_work(const bhsp_batch* b) { return b->mixed && !b->variant_set; }
 
@@ -415,7 +435,7 @@ extern "C" int bhsp_batch_create(bhsp_batch** out, int count, int m_total, int n
     if (e == cudaSuccess) e = cudaMemsetAsync(b->err, 0, sizeof(uint32_t), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(b->ticket, 0, 2 * sizeof(int), st);
     if (e == cudaSuccess) e = launch_partition(d_row_ptr, m_total, nnz_total, 32 * c.seg, b->tile_ptr, st);
-    if (e == cudaSuccess) e = batch_work_build(b, st);
+    if (e == cudaSuccess) e = batch_work_try(b, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
         rc = batch_cuda(b, e, "batch setup");
