@@ -85,8 +85,8 @@ struct bhsp_plan {
     uint32_t* tile_ptr = nullptr;
     int* rec_row = nullptr;
     void* rec_val = nullptr;
-    uint32_t* err = nullptr;  // error word: on the device, or in mapped host memory (plan_map_err)
-    bool err_mapped = false;
+    uint32_t* err = nullptr;  // error word: on the device, or host_err (plan_host_err)
+    uint32_t host_err = 0;
     int* ticket = nullptr;    // [2] the persistent tile kernel's work queue
     int grid_mode = -1;       // the tile kernel's grid: -1 by rule, 0 static, 1 persistent
     int short_rows = 0;     // non-empty rows shorter than one chunk of a lane's slots
@@ -120,16 +120,12 @@ static void plan_release(bhsp_plan* p) {
     cudaFree(p->tile_ptr);
     cudaFree(p->rec_row);
     cudaFree(p->rec_val);
-    if (p->err_mapped)
-        cudaFreeHost(p->err);
-    else
-        cudaFree(p->err);
+    if (p->err != &p->host_err) cudaFree(p->err);
     cudaFree(p->ticket);
     p->tile_ptr = nullptr;
     p->rec_row = nullptr;
     p->rec_val = nullptr;
     p->err = nullptr;
-    p->err_mapped = false;
     p->ticket = nullptr;
 }
 
@@ -284,13 +280,14 @@ static int plan_execute(bhsp_plan* p, const void* val, const void* x, void* y, c
 
 static int plan_check(bhsp_plan* p, cudaStream_t st) {
     uint32_t h = 0;
-    if (!p->err_mapped)
+    volatile uint32_t* const on_host = p->err == &p->host_err ? &p->host_err : nullptr;
+    if (!on_host)
         PLAN_CUDA(p, cudaMemcpyAsync(&h, p->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     PLAN_CUDA(p, cudaStreamSynchronize(st));
-    if (p->err_mapped) h = *static_cast<volatile uint32_t*>(p->err);
+    if (on_host) h = *on_host;
     if (h) {
-        if (p->err_mapped)
-            *static_cast<volatile uint32_t*>(p->err) = 0;
+        if (on_host)
+            *on_host = 0;
         else
             PLAN_CUDA(p, cudaMemsetAsync(p->err, 0, sizeof(uint32_t), st));
         PLAN_CUDA(p, cudaStreamSynchronize(st));
@@ -301,24 +298,14 @@ static int plan_check(bhsp_plan* p, cudaStream_t st) {
     return BHSPARSE_SUCCESS;
 }
 
-// The error word of a handle's plan in mapped host memory, where the host is coherent with the GPU: a
-// check, which every bhsp_run_benchmark ends with, is then a synchronise without a 4-byte copy
-// (10.5 -> 2.0 us; set_x, run and get_y of the 27-point stencil on 80^3, FP64, 119.5 -> 114.7 us).
-// Kernels write the word only when a check of theirs fires.  Not
-// worth its page-locked allocation in a plan of the caller's own, which need not check each product.
-// Without the memory the word stays on the device.
-static void plan_map_err(bhsp_plan* p) {
-    void* word = nullptr;
+// The error word of a handle's plan in the plan itself, where the GPU reads and writes the host's
+// pageable memory coherently: a check, which every bhsp_run_benchmark ends with, is then a synchronise
+// without a 4-byte copy (10.5 -> 2.0 us; set_x, run and get_y of the 27-point stencil on 80^3, FP64,
+// 119.5 -> 114.7 us).  Kernels write the word only when a check of theirs fires.
+static void plan_host_err(bhsp_plan* p) {
     if (!host_direct_access()) return;
-    if (cudaHostAlloc(&word, sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable) !=
-        cudaSuccess) {
-        cudaGetLastError();  // clear the allocation's error
-        return;
-    }
-    *static_cast<uint32_t*>(word) = 0;
     cudaFree(p->err);
-    p->err = static_cast<uint32_t*>(word);
-    p->err_mapped = true;
+    p->err = &p->host_err;
 }
 
 namespace spmv {
@@ -730,7 +717,7 @@ extern "C" int bhsp_prepare_mem(bhsp_spmv* h, int m, int n, int nnz, const int* 
     }
     h->plan = p;
     H_CUDA(h, cudaStreamSynchronize(h->stream));
-    plan_map_err(p);
+    plan_host_err(p);
     h->prepared = true;
     return BHSPARSE_SUCCESS;
 }
