@@ -41,7 +41,7 @@ __global__ void k_batch_calibrate(const int* rec_row, const VecD<1>* rec_val, in
         calibrate_records<PolMixedK<1>>(rec_row, rec_val, nrec, base, y, m, err);
 }
 
-template int batch_work_grid<1>(int);
+template int batch_work_grid<1>(const BatchWork&, int);
 
 template <>
 cudaError_t launch_batch_work<1>(const BatchLaunch& l, const BatchWork& b, int seg,

@@ -3,7 +3,7 @@
 
 namespace spmv {
 
-template int batch_work_grid<2>(int);
+template int batch_work_grid<2>(const BatchWork&, int);
 template cudaError_t launch_batch_work<2>(const BatchLaunch&, const BatchWork&, int, cudaStream_t);
 
 }  // namespace spmv

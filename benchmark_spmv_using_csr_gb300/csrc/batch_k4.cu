@@ -3,7 +3,7 @@
 
 namespace spmv {
 
-template int batch_work_grid<4>(int);
+template int batch_work_grid<4>(const BatchWork&, int);
 template cudaError_t launch_batch_work<4>(const BatchLaunch&, const BatchWork&, int, cudaStream_t);
 
 }  // namespace spmv

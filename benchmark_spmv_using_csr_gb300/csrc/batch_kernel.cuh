@@ -34,7 +34,10 @@ struct BatchArgs {
 };
 
 // ---- tile workers ----
-template <int K, int S>
+// OH, XL2: the kernel variant, chosen from the tile workers' own rows and columns.  With rows of 512
+// near columns between 27-point stencils, half of the non-zeros each, the per-slot form with L2-only
+// gathers takes 107 us at one right-hand side and 168 at two, the variant of these rows 60 and 88.
+template <int K, int S, bool OH, bool XL2>
 __device__ __forceinline__ void batch_tile_workers(const BatchArgs<K>& a, uint32_t* words, int* rowof) {
     using P = PolMixedK<K>;
     const int lane = threadIdx.x & 31;
@@ -53,7 +56,7 @@ __device__ __forceinline__ void batch_tile_workers(const BatchArgs<K>& a, uint32
         t.nnz = __ldg(a.t.row_ptr + d.row1);
         t.row0 = d.row0;
         t.tile_ptr = a.t.tile_ptr + d.at;
-        tile_worker<P, S, false, false, true, true>(t, w, d.first, d.last, words, rowof);
+        tile_worker<P, S, OH, false, XL2, true>(t, w, d.first, d.last, words, rowof);
         __syncwarp();
     }
     if (lane == 0) {
@@ -64,30 +67,42 @@ __device__ __forceinline__ void batch_tile_workers(const BatchArgs<K>& a, uint32
         }
     }
 }
-template <int K, int S>
+template <int K, int S, bool OH, bool XL2>
 __global__ void __launch_bounds__(BATCH_WARPS * 32) k_batch_tiles(BatchArgs<K> a) {
     __shared__ uint32_t s_words[BATCH_WARPS][32];
     __shared__ int s_rowof[BATCH_WARPS][32 * S];
     asm volatile("griddepcontrol.launch_dependents;");
     const int warp = threadIdx.x >> 5;
-    batch_tile_workers<K, S>(a, s_words[warp], s_rowof[warp]);
+    batch_tile_workers<K, S, OH, XL2>(a, s_words[warp], s_rowof[warp]);
 }
 // as k_tiles_persistent_capped: 16 resident warps per SM for 4 and 8 right-hand sides
-template <int K, int S>
+template <int K, int S, bool XL2>
 __global__ void __launch_bounds__(BATCH_WARPS * 32, 16 / BATCH_WARPS)
     k_batch_tiles_capped(BatchArgs<K> a) {
     __shared__ uint32_t s_words[BATCH_WARPS][32];
     __shared__ int s_rowof[BATCH_WARPS][32 * S];
     asm volatile("griddepcontrol.launch_dependents;");
     const int warp = threadIdx.x >> 5;
-    batch_tile_workers<K, S>(a, s_words[warp], s_rowof[warp]);
+    batch_tile_workers<K, S, false, XL2>(a, s_words[warp], s_rowof[warp]);
 }
+template <int K>
+using BatchTilesKernel = void (*)(BatchArgs<K>);
 template <int K, int S>
-constexpr auto batch_tiles_kernel() {
+BatchTilesKernel<K> batch_tiles_variant(bool one_head, bool x_l2) {
     if constexpr (K >= 4)
-        return &k_batch_tiles_capped<K, S>;
+        return x_l2 ? &k_batch_tiles_capped<K, S, true> : &k_batch_tiles_capped<K, S, false>;
+    else if constexpr (K == 2)
+        return x_l2 ? &k_batch_tiles<K, S, false, true> : &k_batch_tiles<K, S, false, false>;
+    else if (one_head)
+        return x_l2 ? &k_batch_tiles<K, S, true, true> : &k_batch_tiles<K, S, true, false>;
     else
-        return &k_batch_tiles<K, S>;
+        return x_l2 ? &k_batch_tiles<K, S, false, true> : &k_batch_tiles<K, S, false, false>;
+}
+template <int K>
+BatchTilesKernel<K> batch_tiles_kernel(const BatchWork& b, int seg) {
+    return seg == 8    ? batch_tiles_variant<K, 8>(b.one_head, b.x_l2)
+           : seg == 16 ? batch_tiles_variant<K, 16>(b.one_head, b.x_l2)
+                       : batch_tiles_variant<K, 32>(b.one_head, b.x_l2);
 }
 
 // ---- row workers ----
@@ -314,19 +329,13 @@ __global__ void __launch_bounds__(BATCH_WARPS * 32, (BatchRows<K, T, NG>::CTAS))
 }
 
 // resident grid of the tile workers' kernel on the current device (0 on failure)
-template <int K, int S>
-int batch_tiles_grid() {
+template <int K>
+int batch_work_grid(const BatchWork& b, int seg) {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, batch_tiles_kernel<K, S>(), BATCH_WARPS * 32, 0) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_tiles_kernel<K>(b, seg),
+                                                      BATCH_WARPS * 32, 0) != cudaSuccess)
         return 0;
     return device_sm_count() * (per_sm > 0 ? per_sm : 1);
-}
-template <int K>
-int batch_work_grid(int seg) {
-    return seg == 8    ? batch_tiles_grid<K, 8>()
-           : seg == 16 ? batch_tiles_grid<K, 16>()
-                       : batch_tiles_grid<K, 32>();
 }
 
 template <int K>
@@ -339,10 +348,7 @@ cudaError_t launch_batch_tiles(const BatchLaunch& l, const BatchWork& b, int seg
     a.t.rec_val = static_cast<VecD<K>*>(b.rec_val);
     a.tiles = b.tiles;
     a.ntiles = b.ntiles;
-    auto* const kernel = seg == 8    ? batch_tiles_kernel<K, 8>()
-                         : seg == 16 ? batch_tiles_kernel<K, 16>()
-                                     : batch_tiles_kernel<K, 32>();
-    kernel<<<b.tiles_grid, BATCH_WARPS * 32, 0, st>>>(a);
+    batch_tiles_kernel<K>(b, seg)<<<b.tiles_grid, BATCH_WARPS * 32, 0, st>>>(a);
     return cudaGetLastError();
 }
 

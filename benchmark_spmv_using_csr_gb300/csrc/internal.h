@@ -181,6 +181,9 @@ constexpr int NLIST_FORMS = 6;
 constexpr ListForm LIST_FORMS_1[NLIST_FORMS] = {{1, 2, 1}, {1, 4, 2}, {1, 7, 3},
                                                 {2, 4, 4}, {2, 7, 5}, {4, 7, -1}};
 constexpr ListForm LIST_FORMS_K[NLIST_FORMS] = {{1, 3, 1}, {1, 7, 2}, {2, 7, 3}, {4, 7, 4}, {8, 7, -1}};
+// The width of the chunks in which the tile kernel takes a lane's slots (tile_kernel.cuh's
+// chunk_width for an x entry of k floats).
+inline int batch_chunk_width(int k, int seg) { return k == 8 ? 2 : (seg == 8 || k == 4) ? 4 : 8; }
 // The two work lists and their kernels' buffers.
 struct BatchWork {
     TileWork* tiles = nullptr;  // [ntiles]
@@ -190,6 +193,8 @@ struct BatchWork {
     int* rec_row = nullptr;  // [ntiles]
     void* rec_val = nullptr;
     int ntiles = 0, nlists = 0, tiles_grid = 0;
+    // the tile workers' kernel variant, from the counts of their own rows and columns
+    bool one_head = false, x_l2 = false;
 };
 // What the work lists need of each block of 256 rows.
 struct BlockStat {
@@ -198,8 +203,11 @@ struct BlockStat {
     int groups[4];  // as RowCounts::groups, over this block
     int eights;     // non-empty rows of a multiple of 8 non-zeros
     int filled;     // non-empty rows
+    int shorts;     // non-empty rows shorter than cw non-zeros
+    uint32_t sampled, near;  // of its every step-th non-zeros, as launch_x_locality counts them
 };
-cudaError_t launch_block_stats(const int* row_ptr, int m, BlockStat* stat, cudaStream_t st);
+cudaError_t launch_block_stats(const int* row_ptr, const int* col, int m, int nnz, int cw, int step,
+                               BlockStat* stat, cudaStream_t st);
 // A run of rows for the tile workers: tiles [t0, t1], boundary t at tile_ptr[at + t - t0].
 struct TileRun {
     int row0, row1, t0, t1, at;

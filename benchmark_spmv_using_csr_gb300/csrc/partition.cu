@@ -169,33 +169,34 @@ __global__ void k_row_counts(const int* __restrict__ row_ptr, int m, int cw,
 // Locality of the columns for the x gathers, on every step-th non-zero: near when its column is
 // within 4 of the previous entry of its row, or of the entry at the same position of the
 // previous row (a stencil's neighbour rows reuse the same x lines).
+__device__ __forceinline__ bool near_column(const int* __restrict__ row_ptr,
+                                            const int* __restrict__ col, int m, int j, int* row) {
+    // the row of non-zero j: the last r with row_ptr[r] <= j (rows 0..m-1)
+    int lo = 0, hi = m - 1;
+    while (lo < hi) {
+        const int mid = (int)(((long long)lo + hi + 1) >> 1);
+        if (__ldg(row_ptr + mid) <= j)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    const int r = *row = lo;
+    const int start = __ldg(row_ptr + r);
+    const int c = __ldg(col + j);
+    if (j > start && abs(c - __ldg(col + j - 1)) <= 4) return true;
+    if (r == 0) return false;
+    const int ps = __ldg(row_ptr + r - 1);
+    return ps + (j - start) < start && abs(c - __ldg(col + ps + (j - start))) <= 4;
+}
 __global__ void k_x_locality(const int* __restrict__ row_ptr, const int* __restrict__ col, int m,
                              int nnz, int step, uint32_t* __restrict__ counts) {
     const long long stride = (long long)gridDim.x * blockDim.x;
     uint32_t seen = 0, near = 0;
     for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s * step < nnz;
          s += stride) {
-        const int j = (int)(s * step);
-        // the row of non-zero j: the last r with row_ptr[r] <= j (rows 0..m-1)
-        int lo = 0, hi = m - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (__ldg(row_ptr + mid) <= j)
-                lo = mid;
-            else
-                hi = mid - 1;
-        }
-        const int r = lo;
-        const int start = __ldg(row_ptr + r);
-        const int c = __ldg(col + j);
-        bool is_near = false;
-        if (j > start) is_near = abs(c - __ldg(col + j - 1)) <= 4;
-        if (!is_near && r > 0) {
-            const int ps = __ldg(row_ptr + r - 1);
-            if (ps + (j - start) < start) is_near = abs(c - __ldg(col + ps + (j - start))) <= 4;
-        }
+        int row = 0;
         ++seen;
-        near += is_near ? 1u : 0u;
+        near += near_column(row_ptr, col, m, (int)(s * step), &row) ? 1u : 0u;
     }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) {
@@ -229,7 +230,7 @@ cudaError_t launch_row_counts(const int* row_ptr, int m, int cw, RowCounts* coun
 }
 
 // One warp per block of 256 rows.
-__global__ void k_block_stats(const int* __restrict__ row_ptr, int m, int nblocks,
+__global__ void k_block_stats(const int* __restrict__ row_ptr, int m, int nblocks, int cw,
                               BlockStat* __restrict__ stat) {
     const int lane = threadIdx.x & 31;
     const int nwarps = gridDim.x * (blockDim.x >> 5);
@@ -242,6 +243,7 @@ __global__ void k_block_stats(const int* __restrict__ row_ptr, int m, int nblock
             const int len = r < m ? __ldg(row_ptr + r + 1) - lo : 0;
             s.filled += __popc(__ballot_sync(SPMV_FULL_MASK, len > 0));
             s.eights += __popc(__ballot_sync(SPMV_FULL_MASK, len > 0 && len % 8 == 0));
+            s.shorts += __popc(__ballot_sync(SPMV_FULL_MASK, len > 0 && len < cw));
             int most = len;
 #pragma unroll
             for (int t = 3, d = 1; t >= 0; --t) {
@@ -254,6 +256,19 @@ __global__ void k_block_stats(const int* __restrict__ row_ptr, int m, int nblock
 #pragma unroll
         for (int t = 0; t < 4; ++t) s.groups[t] = __reduce_add_sync(SPMV_FULL_MASK, s.groups[t]);
         if (lane == 0) stat[b] = s;
+    }
+}
+
+// The locality counts of k_x_locality, per block of 256 rows.
+__global__ void k_block_locality(const int* __restrict__ row_ptr, const int* __restrict__ col,
+                                 int m, int nnz, int step, BlockStat* __restrict__ stat) {
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s * step < nnz;
+         s += stride) {
+        int row = 0;
+        const bool near = near_column(row_ptr, col, m, (int)(s * step), &row);
+        atomicAdd(&stat[row / BATCH_BLOCK].sampled, 1u);
+        if (near) atomicAdd(&stat[row / BATCH_BLOCK].near, 1u);
     }
 }
 
@@ -283,11 +298,15 @@ __global__ void k_run_tiles(const int* __restrict__ row_ptr, const TileRun* __re
     tile_ptr[i] = (uint32_t)(search_right(row_ptr + r.row0, (int)key, m + 1) - 1);
 }
 
-cudaError_t launch_block_stats(const int* row_ptr, int m, BlockStat* stat, cudaStream_t st) {
+cudaError_t launch_block_stats(const int* row_ptr, const int* col, int m, int nnz, int cw, int step,
+                               BlockStat* stat, cudaStream_t st) {
     const int nblocks = (int)(((long long)m + BATCH_BLOCK - 1) / BATCH_BLOCK);
     if (nblocks > 0)
-        k_block_stats<<<grid_for((long long)nblocks * 32, 256, 8), 256, 0, st>>>(row_ptr, m,
-                                                                                nblocks, stat);
+        k_block_stats<<<grid_for((long long)nblocks * 32, 256, 8), 256, 0, st>>>(
+            row_ptr, m, nblocks, cw, stat);
+    if (m > 0 && nnz > 0)
+        k_block_locality<<<grid_for(((long long)nnz + step - 1) / step, 256, 8), 256, 0, st>>>(
+            row_ptr, col, m, nnz, step, stat);
     return cudaGetLastError();
 }
 

@@ -335,7 +335,7 @@ TileArgs<PolMixedK<K>> batch_tile_args(const BatchLaunch& l) {
 
 // batch_k<K>.cu
 template <int K>
-int batch_work_grid(int seg);
+int batch_work_grid(const BatchWork& b, int seg);
 template <int K>
 cudaError_t launch_batch_work(const BatchLaunch& l, const BatchWork& b, int seg, cudaStream_t st);
 template <>

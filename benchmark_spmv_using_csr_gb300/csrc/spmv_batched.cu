@@ -142,6 +142,7 @@ struct bhsp_batch {
     int count = 0, k = 1;
     int m = 0, n = 0, nnz = 0;  // totals of the concatenated block-diagonal matrix
     TileConfig cfg{};
+    bool tpw_by_rule = false;  // the tiles per worker are the rule's, not the caller's
     BatchVariant var{};
     int short_rows = 0, x_sampled = 0, x_near = 0;  // the counts the variant came from
     int ntiles = 0, nworkers = 0, grid = 0;
@@ -228,7 +229,10 @@ static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
     std::vector<BlockStat> stat((size_t)nblocks);
     BlockStat* d_stat = nullptr;
     cudaError_t e = cudaMalloc(&d_stat, sizeof(BlockStat) * (size_t)nblocks);
-    if (e == cudaSuccess) e = launch_block_stats(b->row_ptr, b->m, d_stat, st);
+    const int cw = batch_chunk_width(b->k, b->cfg.seg);
+    const int step = b->nnz > (1 << 20) ? b->nnz / (1 << 20) : 1;
+    if (e == cudaSuccess)
+        e = launch_block_stats(b->row_ptr, b->col, b->m, b->nnz, cw, step, d_stat, st);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(stat.data(), d_stat, sizeof(BlockStat) * (size_t)nblocks,
                             cudaMemcpyDeviceToHost, st);
@@ -265,18 +269,33 @@ static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
         taken[f] = few ? up : f;
         if (few && up >= 0) count[up] += count[f];
     }
-    long long row_nnz = 0;
+    long long row_nnz = 0, shorts = 0, sampled = 0, near = 0;
     for (int i = 0; i < nblocks; ++i) {
         int& f = form[(size_t)i];
+        const BlockStat& s = stat[(size_t)i];
         while (f >= 0 && taken[f] != f) f = taken[f];
-        if (f >= 0) row_nnz += nnz_to(i + 1) - stat[(size_t)i].first;
+        if (f >= 0) {
+            row_nnz += nnz_to(i + 1) - s.first;
+        } else {
+            shorts += s.shorts;
+            sampled += s.sampled;
+            near += s.near;
+        }
     }
     if (4 * row_nnz < b->nnz) return cudaSuccess;
-    // tiles per tile worker (up to 1024 non-zeros), as many as leave every warp several workers: on
-    // the 64-matrix mix 2048 and 4096 non-zeros were 0-5 % slower, on 5 and 16 matrices up to 38 %
+    b->work.one_head = b->k == 1 && one_head_pays(shorts, b->nnz - row_nnz, cw);
+    // (the one-head form gathers through L1 whatever the columns: rows of 300 to 1500 random columns
+    // between stencils, x of 50,000, 216,000 and 1,000,000 entries: 62, 67.5 and 70.0 us through L1,
+    // 80, 68.9 and 69.9 from L2 only)
+    b->work.x_l2 = !b->work.one_head && x_l2_pays(sampled, near);
+    // tiles per tile worker: up to 1024 non-zeros, as many as leave every warp six workers (on the
+    // 128-matrix mix at one right-hand side 199 us; 204 at three workers, 207 at 2048 non-zeros too).
+    // In the one-head form, whose workers cost more to start, up to 2048 and two workers: rows of 512
+    // and of 256 near columns between stencils 67.8 -> 59.7 and 62.2 -> 52.4 us.
+    const bool oh = b->work.one_head;
     const int tpw = (int)std::min<long long>(
-        {b->cfg.tiles_per_worker, std::max(1024 / tile, 1),
-         (int)std::max<long long>((b->nnz - row_nnz) / tile / (6 * warps), 1)});
+        {oh && b->tpw_by_rule ? 4 : b->cfg.tiles_per_worker, std::max((oh ? 2048 : 1024) / tile, 1),
+         (int)std::max<long long>((b->nnz - row_nnz) / tile / ((oh ? 2 : 6) * warps), 1)});
     std::vector<TileWork> tiles;
     std::vector<TileRun> runs;
     std::vector<int> blocks[NLIST_FORMS];
@@ -339,10 +358,10 @@ static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
     cudaFree(d_runs);
     if (e != cudaSuccess) return e;
     switch (b->k) {
-        case 1: w.tiles_grid = batch_work_grid<1>(b->cfg.seg); break;
-        case 2: w.tiles_grid = batch_work_grid<2>(b->cfg.seg); break;
-        case 4: w.tiles_grid = batch_work_grid<4>(b->cfg.seg); break;
-        default: w.tiles_grid = batch_work_grid<8>(b->cfg.seg); break;
+        case 1: w.tiles_grid = batch_work_grid<1>(w, b->cfg.seg); break;
+        case 2: w.tiles_grid = batch_work_grid<2>(w, b->cfg.seg); break;
+        case 4: w.tiles_grid = batch_work_grid<4>(w, b->cfg.seg); break;
+        default: w.tiles_grid = batch_work_grid<8>(w, b->cfg.seg); break;
     }
     b->mixed = w.tiles_grid > 0 && w.nlists > 0;
     return cudaSuccess;
@@ -401,7 +420,7 @@ extern "C" int bhsp_batch_create(bhsp_batch** out, int count, int m_total, int n
     {
         // the kernel variant, as for a single matrix's plan: short rows against the chunk
         // width of the batched kernel, and the locality of about 2^20 sampled columns
-        const int cw = k == 8 ? 2 : (c.seg == 8 || k == 4) ? 4 : 8;  // chunk_width<S, x entry>
+        const int cw = batch_chunk_width(k, c.seg);
         const int step = nnz_total > (1 << 20) ? nnz_total / (1 << 20) : 1;
         struct Counts {
             RowCounts rows;
@@ -424,7 +443,10 @@ extern "C" int bhsp_batch_create(bhsp_batch** out, int count, int m_total, int n
     }
     b->grid = e == cudaSuccess ? batch_grid(k, c, b->var) : 0;
     if (e == cudaSuccess && b->grid <= 0) e = cudaErrorInvalidConfiguration;
-    if (tiles_per_worker <= 0) b->cfg.tiles_per_worker = c.tiles_per_worker = batch_tiles_per_worker(b);
+    if (tiles_per_worker <= 0) {
+        b->tpw_by_rule = true;
+        b->cfg.tiles_per_worker = c.tiles_per_worker = batch_tiles_per_worker(b);
+    }
     b->nworkers = (b->ntiles + c.tiles_per_worker - 1) / c.tiles_per_worker;
     const size_t nw = b->nworkers > 0 ? (size_t)b->nworkers : 1;
     if (e == cudaSuccess) e = cudaMalloc(&b->tile_ptr, sizeof(uint32_t) * ((size_t)b->ntiles + 1));
