@@ -198,11 +198,19 @@ static int batch_cuda(bhsp_batch* b, cudaError_t e, const char* what) {
 // every resident warp has many tiles.  Measured at one right-hand side and 16 non-zeros per lane
 // with 1, 2, 3 and 4 tiles (us): 2 matrices (0.7 tiles per warp) 13.5, 16.6, 18.7, 21.8; 5 (1.8)
 // 27.5, 37.1, 46.6, 57.8; 32 (12) 71, 76, 84, 98; 128 (47) 257, 229, 220, 231; 256 (90) 460, 402,
-// 394, 387.  Power-law matrices at 8 right-hand sides: 26 tiles per warp 344, 314, 311, 313.
+// 394, 387.  From two right-hand sides on, where a warp's tile costs more and so evens out sooner,
+// a worker grows at half as many tiles: power-law matrices at 8 right-hand sides (26 tiles per warp)
+// 344, 314, 311, 313; rows of 300 to 1500 random columns at 8 right-hand sides (8.6) 102, 95, 91, 98,
+// at 4 (10.1) 151, 146, 147, 147; rows of 512 near columns at 8 (10.1) 117, 119, 121, 125.
+// The one-head form (long rows at one right-hand side) spends its time on a worker's start, not on
+// the ends of rows: rows of 300 to 1500 random columns (0.5 tiles per warp) 18.5, 24.6, 26.3, 31.1;
+// (1.6) 27.3, 24.9, 31.2, 37.3; (2.6) 36.4, 35.4, 31.6, 37.4; (4.2) 48.2, 49.5, 48.4, 45.6; (5.8)
+// 66.5, 65.7, 66.6, 63.0; (13.5) 144, 140, 137, 130.
 static int batch_tiles_per_worker(const bhsp_batch* b) {
     const long long warps = (long long)b->grid * b->cfg.warps_per_cta;
+    if (b->var.one_head) return b->ntiles >= 4 * warps ? 4 : 1;
     int tpw = 1;
-    while (tpw < 4 && b->ntiles >= (7LL << tpw) * warps) ++tpw;
+    while (tpw < 4 && b->ntiles >= ((b->k == 1 ? 14LL : 7LL) << (tpw - 1)) * warps) ++tpw;
     return tpw;
 }
 
