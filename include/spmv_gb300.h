@@ -220,8 +220,8 @@ int bhsp_batch_create(bhsp_batch** out, int count, int m_total, int n_total, int
                       const int* d_row_ptr, const int* d_col_idx, int k, int seg,
                       int tiles_per_worker, int warps_per_cta, void* stream);
 /* y = A.x for all matrices and right-hand sides, enqueued on `stream`.  use_graph != 0 replays a
- * CUDA graph of the batch's kernels (captured on the
- * first call and again whenever the buffers change); use_graph == 0 launches them directly.
+ * CUDA graph of the batch's kernels, captured when a set of buffers comes a second time in a row;
+ * other calls, and all with use_graph == 0, launch the kernels directly.
  * d_val 32-byte aligned, d_x / d_y aligned to 4*k bytes. */
 int bhsp_batch_execute(bhsp_batch* b, const float* d_val, const float* d_x, float* d_y,
                        int use_graph, void* stream);

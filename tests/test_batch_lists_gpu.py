@@ -98,3 +98,49 @@ def test_tile_workers_variants_bit_exact(cuda_ok, k, seg, spread):
         b.check()
         assert (y.cpu().numpy() == want).all(), use_graph
     b.close()
+
+
+@pytest.mark.parametrize("k", [1, 8])
+def test_changing_buffers_cost_no_capture_per_call(cuda_ok, k):
+    """Two x / y pairs in turn with use_graph: exact on both, and a call takes at most 1.25 times what
+    a direct launch takes, and 3 us (a capture and instantiation per call would be 15 us and more);
+    the same pair over and over is a graph replay, exact too, also after the other pair."""
+    import torch
+    rng = np.random.default_rng(k)
+    mats = [gen.stencil2d(80, 80), gen.powerlaw(5000, seed=2), gen.blockdiag(4096, 4096, 32)]
+    for a in mats:
+        a.val = rng.integers(-4, 5, a.nnz).astype(np.float64)
+    b = batch.Batch(mats, k=k)
+    row = np.repeat(np.arange(b.m), np.diff(b.cat["row_ptr"]))
+    pairs = []
+    for _ in range(2):
+        x = rng.integers(-4, 5, (b.n, k)).astype(np.float64)
+        want = np.stack([np.bincount(row, b.cat["val"] * x[b.cat["col"], i], b.m) for i in range(k)], 1)
+        pairs.append((torch.from_numpy(x.astype(np.float32)).cuda(),
+                      torch.empty((b.m, k), dtype=torch.float32, device="cuda"), want))
+
+    def per_call(use_graph, turn):
+        out = []
+        for _ in range(6):
+            torch.cuda.synchronize()
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            for i in range(40):
+                x, y, _ = pairs[i % 2 if turn else 0]
+                b.execute(x, y, use_graph=use_graph)
+            e1.record()
+            torch.cuda.synchronize()
+            out.append(e0.elapsed_time(e1) * 25)
+        return sorted(out[1:])[2]
+
+    direct = per_call(False, True)
+    turns = per_call(True, True)
+    per_call(True, False)
+    for i in (0, 1, 1, 1, 0, 0, 1, 0):
+        x, y, want = pairs[i]
+        y.fill_(float("nan"))
+        b.execute(x, y)
+        b.check()
+        assert (y.cpu().numpy() == want).all(), i
+    b.close()
+    assert turns <= 1.25 * direct + 3.0, (turns, direct)
