@@ -509,8 +509,9 @@ static cudaError_t enqueue(bhsp_batch* b, const BatchLaunch& l, cudaStream_t st)
     }
 }
 
-extern "C" int bhsp_batch_execute(bhsp_batch* b, const float* d_val, const float* d_x, float* d_y,
-                                  int use_graph, void* stream) {
+// capture_now: a new set of buffers is captured at once (the tuner, which times replays)
+static int batch_execute(bhsp_batch* b, const float* d_val, const float* d_x, float* d_y,
+                         int use_graph, bool capture_now, void* stream) {
     if (!b || !d_y || (b->nnz > 0 && (!d_val || !d_x))) return BHSPARSE_INVALID_ARGUMENT;
     if (reinterpret_cast<uintptr_t>(d_val) % 32 != 0 ||
         reinterpret_cast<uintptr_t>(d_x) % (4 * b->k) != 0 || reinterpret_cast<uintptr_t>(d_y) % (4 * b->k) != 0)
@@ -523,7 +524,7 @@ extern "C" int bhsp_batch_execute(bhsp_batch* b, const float* d_val, const float
     // 42 -> 28.5 on 5 (3 kernels), 117 -> 112 on 64 (7 kernels, one right-hand side); the first call
     // on new buffers, waited for, 50 -> 22, 98 -> 56 and 180 -> 126.
     const bhsp_batch::Buffers now{d_val, d_x, d_y};
-    const bool again = b->last == now;
+    const bool again = capture_now || b->last == now;
     if (use_graph) b->last = now;
     const bool ready = b->exec && b->captured == now;
     if (!use_graph || (!ready && !again)) {
@@ -552,6 +553,11 @@ extern "C" int bhsp_batch_execute(bhsp_batch* b, const float* d_val, const float
     }
     cudaError_t e = cudaGraphLaunch(b->exec, st);
     return e == cudaSuccess ? BHSPARSE_SUCCESS : batch_cuda(b, e, "graph launch");
+}
+
+extern "C" int bhsp_batch_execute(bhsp_batch* b, const float* d_val, const float* d_x, float* d_y,
+                                  int use_graph, void* stream) {
+    return batch_execute(b, d_val, d_x, d_y, use_graph, false, stream);
 }
 
 extern "C" int bhsp_batch_check(bhsp_batch* b, void* stream) {
@@ -681,12 +687,12 @@ extern "C" int bhsp_batch_autotune(int count, int m_total, int n_total, int nnz_
                                kBatchCands[i].seg, kBatchCands[i].tpw, kBatchCands[i].warps,
                                stream);
         if (rc) break;
-        for (int w = 0; w < warmup && rc == 0; ++w) rc = bhsp_batch_execute(b, d_val, d_x, d_y, 1, stream);
+        for (int w = 0; w < warmup && rc == 0; ++w) rc = batch_execute(b, d_val, d_x, d_y, 1, true, stream);
         for (int r = 0; r < reps && rc == 0; ++r) {
             if (flush && cudaMemsetAsync(flush, r & 0xff, flush_bytes, st) != cudaSuccess)
                 rc = BHSPARSE_CUDA_ERROR;
             if (!rc && cudaEventRecord(e0, st) != cudaSuccess) rc = BHSPARSE_CUDA_ERROR;
-            if (!rc) rc = bhsp_batch_execute(b, d_val, d_x, d_y, 1, stream);
+            if (!rc) rc = batch_execute(b, d_val, d_x, d_y, 1, true, stream);
             if (!rc && cudaEventRecord(e1, st) != cudaSuccess) rc = BHSPARSE_CUDA_ERROR;
             if (!rc && cudaEventSynchronize(e1) != cudaSuccess) rc = BHSPARSE_CUDA_ERROR;
             if (!rc && cudaEventElapsedTime(&t[(size_t)r], e0, e1) != cudaSuccess)
