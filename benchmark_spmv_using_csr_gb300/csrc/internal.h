@@ -193,6 +193,7 @@ struct BatchWork {
     int* rec_row = nullptr;  // [ntiles]
     void* rec_val = nullptr;
     int ntiles = 0, nlists = 0, tiles_grid = 0;
+    int tpw = 0;  // tiles per tile worker
     // the tile workers' kernel variant, from the counts of their own rows and columns
     bool one_head = false, x_l2 = false;
 };

@@ -308,6 +308,7 @@ static cudaError_t batch_work_build(bhsp_batch* b, cudaStream_t st) {
     const int tpw = (int)std::min<long long>(
         {oh && b->tpw_by_rule ? 4 : b->cfg.tiles_per_worker, std::max((oh ? 2048 : 1024) / tile, 1),
          (int)std::max<long long>((b->nnz - row_nnz) / tile / ((oh ? 2 : 6) * warps), 1)});
+    b->work.tpw = tpw;
     std::vector<TileWork> tiles;
     std::vector<TileRun> runs;
     std::vector<int> blocks[NLIST_FORMS];
@@ -681,12 +682,33 @@ extern "C" int bhsp_batch_autotune(int count, int m_total, int n_total, int nnz_
     int rc = BHSPARSE_SUCCESS, best_i = -1;
     float best_ms = 0.f;
     std::vector<float> t((size_t)reps);
+    // Over work lists several candidates are one schedule (the lists' kernels have 4 warps per CTA and
+    // a bound on a worker's tiles; without tile workers there is none): it is timed once, so that the
+    // pick is not the luckiest of several runs of it.
+    struct Lists {
+        bool used;
+        int seg, tpw;
+    } lists[kNumBatchCands] = {};
     for (int i = 0; i < kNumBatchCands && rc == BHSPARSE_SUCCESS; ++i) {
         bhsp_batch* b = nullptr;
         rc = bhsp_batch_create(&b, count, m_total, n_total, nnz_total, d_row_ptr, d_col_idx, k,
                                kBatchCands[i].seg, kBatchCands[i].tpw, kBatchCands[i].warps,
                                stream);
         if (rc) break;
+        lists[i].used = batch_takes_work(b);
+        if (lists[i].used && b->work.ntiles > 0) {
+            lists[i].seg = b->cfg.seg;
+            lists[i].tpw = b->work.tpw;
+        }
+        int same = 0;
+        while (same < i && !(lists[i].used && lists[same].used && lists[same].seg == lists[i].seg &&
+                             lists[same].tpw == lists[i].tpw))
+            ++same;
+        if (same < i) {
+            ms_out[i] = ms_out[same];
+            bhsp_batch_destroy(b);
+            continue;
+        }
         for (int w = 0; w < warmup && rc == 0; ++w) rc = batch_execute(b, d_val, d_x, d_y, 1, true, stream);
         for (int r = 0; r < reps && rc == 0; ++r) {
             if (flush && cudaMemsetAsync(flush, r & 0xff, flush_bytes, st) != cudaSuccess)

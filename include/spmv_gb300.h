@@ -244,7 +244,9 @@ int bhsp_batch_set_variant(bhsp_batch* b, int one_head, int l2_only);
  * times bhsp_batch_execute (graph replay; `warmup` untimed runs, then the median of `reps`
  * CUDA-event-timed runs, each after a write of twice the L2 size) on the caller's buffers,
  * writing ms_out[bhsp_batch_tune_num_candidates()] and the fastest's index to *best; pass the
- * pick to bhsp_batch_create.  Synchronous. */
+ * pick to bhsp_batch_create.  Candidates that are one schedule for this batch (its row blocks have
+ * none, and its tile workers take 4 warps per CTA and a bounded number of tiles) are timed once and
+ * get one time.  Synchronous. */
 int bhsp_batch_tune_num_candidates(void);
 int bhsp_batch_tune_candidate(int index, int* seg, int* tiles_per_worker, int* warps_per_cta);
 int bhsp_batch_autotune(int count, int m_total, int n_total, int nnz_total, const int* d_row_ptr,

@@ -144,3 +144,23 @@ def test_changing_buffers_cost_no_capture_per_call(cuda_ok, k):
         assert (y.cpu().numpy() == want).all(), i
     b.close()
     assert turns <= 1.25 * direct + 3.0, (turns, direct)
+
+
+@pytest.mark.parametrize("k", [1, 8])
+def test_autotune_times_one_schedule_once(cuda_ok, k):
+    """Candidates that differ only in what work lists do not use have one time: the warps per CTA
+    where tile workers run beside row blocks, everything where there are none; the pick is the first
+    of the fastest."""
+    import torch
+    stencil = gen.stencil3d(20, 21, 22)
+    for mats, tiles in (([stencil, gen.powerlaw(20_000, seed=3)] * 2, True), ([stencil] * 2, False)):
+        b = batch.Batch(mats, k=k)
+        x = torch.rand(b.n, k, device="cuda")
+        y = torch.empty(b.m, k, device="cuda")
+        ms, best = batch.autotune(b, x, y, warmup=1, reps=3)
+        cands = batch.tune_candidates()
+        for i, (seg, tpw, warps) in enumerate(cands):
+            assert ms[i] == ms[cands.index((seg, tpw, 4))]
+            assert tiles or ms[i] == ms[0]
+        assert best == int(np.argmin(ms))
+        b.close()
