@@ -119,13 +119,13 @@ struct BatchRowArgs {
     const int* __restrict__ col;
     const float* __restrict__ val;
     const VecF<K>* __restrict__ x;
-    VecF<K>* __restrict__ y;
+    VecF<K>* y;
     uint32_t* err;
     int m, nnz;
     const int* __restrict__ blocks;  // first rows of the blocks of BATCH_BLOCK rows to do
     int ppw, nworkers;               // a worker is ppw consecutive passes of a block
-    const int* __restrict__ rec_row;  // the tile workers' carry records, added by the last kernel
-    const VecD<K>* __restrict__ rec_val;
+    const int* rec_row;  // the tile workers' carry records, added by the last kernel
+    const VecD<K>* rec_val;
     int nrec;
 };
 template <int K, int T, int NG>

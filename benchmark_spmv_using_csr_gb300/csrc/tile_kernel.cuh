@@ -774,11 +774,13 @@ __device__ __forceinline__ R rec_shfl(const R& v, int d) {
 // dense-row matrix of 1M rows 61.2 us per product in FP64 where it now takes 58.8, the power-law
 // matrix of 700K rows 61.3 -> 57.9 (mixed FP32), and, at 256 non-zeros per worker (4000 records in
 // the longest run), 114 -> 62 us.
+// The kernel that calls this begins while the one that writes the records and y still runs, and waits
+// for it (griddepcontrol.wait) first.  So none of the three pointers is declared __restrict__: const
+// __restrict__ data may be read by the non-coherent load, which is defined only for data that nobody
+// writes during the whole kernel, and ahead of the wait.
 template <class P>
-__device__ __forceinline__ void calibrate_records(const int* __restrict__ rec_row,
-                                                  const typename P::Rec* __restrict__ rec_val,
-                                                  int nworkers, int base,
-                                                  typename P::YT* __restrict__ y, int m,
+__device__ __forceinline__ void calibrate_records(const int* rec_row, const typename P::Rec* rec_val,
+                                                  int nworkers, int base, typename P::YT* y, int m,
                                                   uint32_t* err) {
     using Rec = typename P::Rec;
     using YT = typename P::YT;
@@ -848,10 +850,9 @@ __device__ __forceinline__ void calibrate_records(const int* __restrict__ rec_ro
 
 // Also zeroes the leading empty rows, which lie in no tile span (the reference never writes them).
 template <class P>
-__global__ void k_calibrate(const int* __restrict__ rec_row,
-                            const typename P::Rec* __restrict__ rec_val, int nworkers,
-                            typename P::YT* __restrict__ y, const uint32_t* __restrict__ tile_ptr,
-                            int m, uint32_t* err) {
+__global__ void k_calibrate(const int* rec_row, const typename P::Rec* rec_val, int nworkers,
+                            typename P::YT* y, const uint32_t* __restrict__ tile_ptr, int m,
+                            uint32_t* err) {
     using YT = typename P::YT;
     // launched as a programmatic dependent of the tile kernel: wait until that grid has
     // completed and its records and y are visible (returns at once for an ordinary launch)
