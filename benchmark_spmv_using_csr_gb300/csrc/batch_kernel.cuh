@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(BATCH_WARPS * 32, (BatchRows<K, T, NG>::CTAS))
         r.rot = ROT ? ((off >> 5) * T) % max(len, 1) : 0;
         if (L::STAGES == 2) fill_stage(stage ^ 1);
         if (!mbar_wait_bounded(bar + stage, phases >> stage & 1u)) {
-            if (lane == 0) atomicOr(a.err, ERR_WAIT_TIMEOUT);
+            if (lane == 0) raise_error(a.err, ERR_WAIT_TIMEOUT);
             // once more for the copies in flight, then give up
             mbar_wait_bounded(bar + stage, phases >> stage & 1u);
             if (L::STAGES == 2 && row >= 0) mbar_wait_bounded(bar + (stage ^ 1), phases >> (stage ^ 1) & 1u);

@@ -280,17 +280,18 @@ static int plan_execute(bhsp_plan* p, const void* val, const void* x, void* y, c
 
 static int plan_check(bhsp_plan* p, cudaStream_t st) {
     uint32_t h = 0;
-    volatile uint32_t* const on_host = p->err == &p->host_err ? &p->host_err : nullptr;
+    const bool on_host = p->err == &p->host_err;
     if (!on_host)
         PLAN_CUDA(p, cudaMemcpyAsync(&h, p->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     PLAN_CUDA(p, cudaStreamSynchronize(st));
-    if (on_host) h = *on_host;
+    // one exchange: a bit that a kernel on another stream sets now is in h or stays for the next check
+    if (on_host && __atomic_load_n(&p->host_err, __ATOMIC_ACQUIRE))
+        h = __atomic_exchange_n(&p->host_err, 0u, __ATOMIC_ACQ_REL);
     if (h) {
-        if (on_host)
-            *on_host = 0;
-        else
+        if (!on_host) {
             PLAN_CUDA(p, cudaMemsetAsync(p->err, 0, sizeof(uint32_t), st));
-        PLAN_CUDA(p, cudaStreamSynchronize(st));
+            PLAN_CUDA(p, cudaStreamSynchronize(st));
+        }
         char buf[96];
         snprintf(buf, sizeof buf, "device-side check failed (error word 0x%x)", h);
         return plan_fail(p, BHSPARSE_DEVICE_CHECK_FAILED, buf);
@@ -755,6 +756,11 @@ extern "C" int bhsp_check(bhsp_spmv* h) {
     int rc = plan_check(h->plan, h->stream);
     if (rc) h->last_error = h->plan->last_error;
     return rc;
+}
+
+// For tests (not in the public header): the handle's error word where it is host memory, else null.
+extern "C" uint32_t* bhsp_debug_host_error_word(bhsp_spmv* h) {
+    return h && h->plan && h->plan->err == &h->plan->host_err ? h->plan->err : nullptr;
 }
 
 extern "C" int bhsp_run_benchmark(bhsp_spmv* h) {

@@ -22,6 +22,10 @@ enum : uint32_t {
     ERR_WAIT_TIMEOUT = 1u << 3,  // an mbarrier wait ran out of its iteration budget
 };
 
+// Sets bits of the error word.  System scope: a handle's word is host memory, which the CPU reads and
+// clears (an exchange) while kernels on other streams may be running.
+__device__ __forceinline__ void raise_error(uint32_t* err, uint32_t bits) { atomicOr_system(err, bits); }
+
 // ---- shared-memory addresses, mbarriers and bulk (TMA) copies ----
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));

@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(ROW_WARPS * 32, (row_min_ctas<P, NG>())) k_row
         const int top = __reduce_max_sync(SPMV_FULL_MASK, len);
         const int low = __reduce_min_sync(SPMV_FULL_MASK, len);
         if (!mbar_wait_bounded(bar, phase)) {
-            if (lane == 0) atomicOr(a.err, ERR_WAIT_TIMEOUT);
+            if (lane == 0) raise_error(a.err, ERR_WAIT_TIMEOUT);
             mbar_wait_bounded(bar, phase);  // once more for the copies in flight, then give up
             break;
         }

@@ -132,7 +132,7 @@ __device__ __forceinline__ void store_row(YT* y, int m, int row, YT v, uint32_t*
     if ((unsigned)row < (unsigned)m)
         y[row] = v;
     else
-        atomicOr(err, ERR_BAD_TILE);
+        raise_error(err, ERR_BAD_TILE);
 }
 
 // Loops over the lanes of a warp that run once per tile or less: fully unrolled for scalar
@@ -658,7 +658,7 @@ __device__ __forceinline__ void persistent_workers(const TileArgs<P>& a, int tpw
         w = __shfl_sync(SPMV_FULL_MASK, w, 0);
         if (w >= nworkers) break;
         if (w < 0) {  // cannot happen with the ticket at zero before the launch
-            if (lane == 0) atomicOr(a.err, ERR_QUEUE);
+            if (lane == 0) raise_error(a.err, ERR_QUEUE);
             break;
         }
         tile_worker<P, S, OH, MID, XL2>(a, w, w * tpw, min((w + 1) * tpw, ntiles), s_words_w,
@@ -844,7 +844,7 @@ __device__ __forceinline__ void calibrate_records(const int* rec_row, const type
         if (r < m)
             y[r] = P::out_rec(P::rec_add(P::rec_of_y(y[r]), acc));
         else
-            atomicOr(err, ERR_BAD_TILE);
+            raise_error(err, ERR_BAD_TILE);
     }
 }
 

@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1)
         // the copies of tiles [t_fail, issued) may still be in flight; each must land (bounded
         // wait) before the warp's shared memory is released
         if (lane == 0) {
-            atomicOr(a.err, ERR_WAIT_TIMEOUT);
+            raise_error(a.err, ERR_WAIT_TIMEOUT);
             if (!rec_written) a.rec_row[worker] = -1;
         }
         for (int t = t_fail; t < issued; ++t) {

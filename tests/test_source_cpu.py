@@ -19,3 +19,12 @@ def test_carry_records_are_not_read_as_constant_data():
     for name, text in _sources():
         found = re.findall(r"const\s[^;,(){}]*__restrict__\s+rec_(?:row|val)\b", text)
         assert not found, (name, found)
+
+
+def test_kernels_raise_errors_at_system_scope():
+    """A handle's error word is host memory: kernels set its bits through raise_error, which is atomic
+    for the CPU too."""
+    for name, text in _sources():
+        assert not re.findall(r"\batomicOr\(\s*(?:a\.)?err\b", text), name
+    common = dict(_sources())["common.cuh"]
+    assert re.search(r"void raise_error\([^)]*\) \{ atomicOr_system\(", common)
