@@ -733,7 +733,9 @@ def schedule_choice(h, tuning) -> dict:
     cfg = tuple(h.get_config())
     key = ",".join(map(str, cfg))
     t = tuning["table_ms"].get(key) if tuning else None
-    return {"schedule": list(cfg), "source": SOURCE_NAMES.get(src, str(src)),
+    lanes, slots = h.kernel()
+    return {"kernel": f"rows ({lanes} lanes x {slots} slots, no schedule)" if lanes else "tiles",
+            "schedule": list(cfg), "source": SOURCE_NAMES.get(src, str(src)),
             "confidence": round(conf, 4),
             "frac_of_autotuner_best": round(tuning["best_ms"] / t, 4) if t else None}
 
@@ -857,6 +859,9 @@ def measure_batched(args) -> dict:
                         "normwise_err_vs_fp64_oracle_max": worst, "launches": info["launches"],
                         "graph": True, "schedule": tb["pick"],
                         "variant": {"one_head": info["one_head"], "x_l2_only": info["x_l2_only"]},
+                        "lists": {key: info[key] for key in ("row_lists", "tile_workers",
+                                                             "workers_one_head",
+                                                             "workers_x_l2_only")},
                         "default_schedule_ms": tb["table_ms"][dflt],
                         "tuning_table_ms": tb["table_ms"]}
         b.close()

@@ -39,6 +39,7 @@ SIGNATURES = {
     "bhsp_set_tuner": (c_int, [c_void_p, c_char_p]),
     "bhsp_get_schedule_source": (c_int, [c_void_p, P_int, ctypes.POINTER(ctypes.c_float)]),
     "bhsp_get_config": (c_int, [c_void_p, P_int, P_int, P_int, P_int]),
+    "bhsp_get_kernel": (c_int, [c_void_p, P_int, P_int]),
     "bhsp_set_x": (c_int, [c_void_p, c_void_p]),
     "bhsp_run_stream": (c_int, [c_void_p, c_int, c_void_p, c_void_p]),
     "bhsp_run_async": (c_int, [c_void_p, c_void_p]),
@@ -53,6 +54,7 @@ SIGNATURES = {
     "bhsp_plan_execute_phase": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int]),
     "bhsp_plan_check": (c_int, [c_void_p, c_void_p]),
     "bhsp_plan_launches": (c_int, [c_void_p]),
+    "bhsp_plan_kernel": (c_int, [c_void_p, P_int, P_int]),
     "bhsp_plan_tiles": (c_int, [c_void_p, P_void, P_int, P_int]),
     "bhsp_plan_chunk_form": (c_int, [c_void_p, P_int, P_int]),
     "bhsp_plan_gather_path": (c_int, [c_void_p, P_int, P_int, P_int]),
@@ -73,6 +75,7 @@ SIGNATURES = {
     "bhsp_batch_info": (c_int, [c_void_p, P_int, P_int, P_int, P_int]),
     "bhsp_batch_last_error": (c_char_p, [c_void_p]),
     "bhsp_batch_variant": (c_int, [c_void_p, P_int, P_int]),
+    "bhsp_batch_lists": (c_int, [c_void_p, P_int, P_int, P_int, P_int]),
     "bhsp_batch_set_variant": (c_int, [c_void_p, c_int, c_int]),
     "bhsp_batch_tune_num_candidates": (c_int, []),
     "bhsp_batch_tune_candidate": (c_int, [c_int, P_int, P_int, P_int]),

@@ -140,6 +140,15 @@ class BhsparseSpmvCuda:
                                 ctypes.byref(d))
         return a.value, b.value, c.value, d.value
 
+    def kernel(self) -> tuple[int, int]:
+        """(lanes per row, non-zeros per lane) of the row kernel the prepared matrix runs, (0, 0)
+        for the tile kernel at the schedule of get_config()."""
+        lanes, slots = ctypes.c_int(), ctypes.c_int()
+        rc = self._L.bhsp_get_kernel(self._h, ctypes.byref(lanes), ctypes.byref(slots))
+        if rc != BHSPARSE_SUCCESS:
+            raise SpmvError(rc, "bhsp_get_kernel failed (before prepare_mem?)")
+        return lanes.value, slots.value
+
     def set_x(self, x) -> int:
         xx = np.ascontiguousarray(x, dtype=host_dtype(self.value_type))
         rc = self._L.bhsp_set_x(self._h, _ptr(xx))
@@ -237,6 +246,13 @@ class Plan:
     @property
     def launches(self) -> int:
         return int(self._L.bhsp_plan_launches(self._p))
+
+    def kernel(self) -> tuple[int, int]:
+        """(lanes per row, non-zeros per lane) of the row kernel that execute runs, (0, 0) for the
+        tile kernel."""
+        lanes, slots = ctypes.c_int(), ctypes.c_int()
+        self._L.bhsp_plan_kernel(self._p, ctypes.byref(lanes), ctypes.byref(slots))
+        return lanes.value, slots.value
 
     def tiles(self) -> tuple[int, int, int]:
         tp, nt, tn = ctypes.c_void_p(), ctypes.c_int(), ctypes.c_int()

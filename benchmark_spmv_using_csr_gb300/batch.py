@@ -99,12 +99,19 @@ class Batch:
             raise RuntimeError(f"batched kernel check failed ({rc}): {self.last_error}")
 
     def info(self) -> dict:
+        """bhsp_batch_info, the variant of the tile kernel over the whole batch, and, where the batch
+        takes work lists instead (row_lists > 0), their kernels and the tile workers' variant."""
         v = [ctypes.c_int() for _ in range(4)]
         lib().bhsp_batch_info(self._b, *[ctypes.byref(c) for c in v])
         out = dict(zip(("ntiles", "nworkers", "grid", "launches"), (c.value for c in v)))
         oh, l2 = ctypes.c_int(), ctypes.c_int()
         lib().bhsp_batch_variant(self._b, ctypes.byref(oh), ctypes.byref(l2))
         out.update(one_head=bool(oh.value), x_l2_only=bool(l2.value))
+        lists, workers = ctypes.c_int(), ctypes.c_int()
+        lib().bhsp_batch_lists(self._b, ctypes.byref(lists), ctypes.byref(workers),
+                               ctypes.byref(oh), ctypes.byref(l2))
+        out.update(row_lists=lists.value, tile_workers=workers.value,
+                   workers_one_head=bool(oh.value), workers_x_l2_only=bool(l2.value))
         return out
 
     def set_variant(self, one_head: bool | None = None, l2_only: bool | None = None) -> None:

@@ -390,6 +390,14 @@ extern "C" int bhsp_plan_launches(const bhsp_plan* p) {
     return p->m == 0 ? 0 : (p->nworkers > 0 && !plan_takes_rows(p) ? 2 : 1);
 }
 
+extern "C" int bhsp_plan_kernel(const bhsp_plan* p, int* lanes, int* slots) {
+    if (!p) return BHSPARSE_INVALID_ARGUMENT;
+    const bool rows = plan_takes_rows(p);
+    if (lanes) *lanes = rows ? p->rows.lanes : 0;
+    if (slots) *slots = rows ? 4 * p->rows.groups : 0;
+    return BHSPARSE_SUCCESS;
+}
+
 extern "C" int bhsp_plan_tiles(const bhsp_plan* p, const uint32_t** d_tile_ptr, int* ntiles,
                                int* tile_nnz) {
     if (!p) return BHSPARSE_INVALID_ARGUMENT;
@@ -586,6 +594,12 @@ extern "C" int bhsp_get_config(const bhsp_spmv* h, int* seg, int* tpw, int* warp
     return BHSPARSE_SUCCESS;
 }
 
+extern "C" int bhsp_get_kernel(const bhsp_spmv* h, int* lanes, int* slots) {
+    if (!h) return BHSPARSE_INVALID_ARGUMENT;
+    if (!h->prepared) return BHSPARSE_NOT_PREPARED;
+    return bhsp_plan_kernel(h->plan, lanes, slots);
+}
+
 static void stream_release(bhsp_spmv* h) {
     for (int i = 0; i < 2; ++i) {
         cudaFree(h->d_xs[i]);
@@ -696,15 +710,6 @@ extern "C" int bhsp_prepare_mem(bhsp_spmv* h, int m, int n, int nnz, const int* 
         }
         h->cfg = make_config(c[0], c[1], c[2], c[3], h->vt);
     }
-    if (const char* lg = std::getenv("BHSP_LOG_SCHEDULE"); lg && *lg && *lg != '0') {
-        static const char* const kSource[] = {"the caller (bhsp_set_config)", "the fixed default",
-                                              "the learned network", "the autotune sweep"};
-        const int src = h->cfg_user ? BHSP_SCHEDULE_CALLER : h->sched_source;
-        std::fprintf(stderr,
-                     "bhsp: m=%d nnz=%d schedule (%d, %d, %d, %d) from %s (confidence %.3f)\n", m,
-                     nnz, h->cfg.seg, h->cfg.tiles_per_worker, h->cfg.warps_per_cta, h->cfg.stages,
-                     kSource[src & 3], (double)(h->cfg_user ? 0.f : h->sched_conf));
-    }
     rc = upload_values(h, h->d_y, y, (size_t)m, false);
     if (rc) return rc;
     bhsp_plan* p = nullptr;
@@ -717,6 +722,19 @@ extern "C" int bhsp_prepare_mem(bhsp_spmv* h, int m, int n, int nnz, const int* 
         return rc;
     }
     h->plan = p;
+    if (const char* lg = std::getenv("BHSP_LOG_SCHEDULE"); lg && *lg && *lg != '0') {
+        static const char* const kSource[] = {"the caller (bhsp_set_config)", "the fixed default",
+                                              "the learned network", "the autotune sweep"};
+        const int src = h->cfg_user ? BHSP_SCHEDULE_CALLER : h->sched_source;
+        char rows[96] = "";
+        if (plan_takes_rows(p))
+            snprintf(rows, sizeof rows, ", not used: row kernel, %d lanes to a row, %d slots to a lane",
+                     p->rows.lanes, 4 * p->rows.groups);
+        std::fprintf(stderr,
+                     "bhsp: m=%d nnz=%d schedule (%d, %d, %d, %d) from %s (confidence %.3f)%s\n", m,
+                     nnz, h->cfg.seg, h->cfg.tiles_per_worker, h->cfg.warps_per_cta, h->cfg.stages,
+                     kSource[src & 3], (double)(h->cfg_user ? 0.f : h->sched_conf), rows);
+    }
     H_CUDA(h, cudaStreamSynchronize(h->stream));
     plan_host_err(p);
     h->prepared = true;

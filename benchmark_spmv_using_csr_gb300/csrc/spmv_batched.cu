@@ -609,6 +609,17 @@ extern "C" int bhsp_batch_variant(const bhsp_batch* b, int* one_head, int* l2_on
     return BHSPARSE_SUCCESS;
 }
 
+extern "C" int bhsp_batch_lists(const bhsp_batch* b, int* row_lists, int* tile_workers, int* one_head,
+                                int* l2_only) {
+    if (!b) return BHSPARSE_INVALID_ARGUMENT;
+    const BatchWork w = batch_takes_work(b) ? b->work : BatchWork{};
+    if (row_lists) *row_lists = w.nlists;
+    if (tile_workers) *tile_workers = w.ntiles;
+    if (one_head) *one_head = w.ntiles > 0 && w.one_head ? 1 : 0;
+    if (l2_only) *l2_only = w.ntiles > 0 && w.x_l2 ? 1 : 0;
+    return BHSPARSE_SUCCESS;
+}
+
 extern "C" int bhsp_batch_set_variant(bhsp_batch* b, int one_head, int l2_only) {
     if (!b || one_head < -1 || one_head > 1 || l2_only < -1 || l2_only > 1 ||
         (one_head == 1 && b->k != 1))

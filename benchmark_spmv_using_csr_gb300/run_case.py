@@ -5,15 +5,16 @@ launch).
     python -m benchmark_spmv_using_csr_gb300.run_case --workload stencil27_160 \
         --form mixed_f32 [--config S TPW WARPS STAGES] [--steps 5] [--warmup 2]
 
-Without --config the schedule is the one prepare_mem chooses.  Each step is the tile kernel
-followed by the calibration kernel, with a 256 MiB write before it so that it starts with the
+Without --config the schedule is the one prepare_mem chooses, or the matrix takes the row kernel.
+Each step is the tile kernel followed by the calibration kernel, or the row kernel, with a 256 MiB write before it so that it starts with the
 matrix out of L2; steps are timed with CUDA events.
 
     python -m benchmark_spmv_using_csr_gb300.run_case --batched K [--config S TPW WARPS 0]
 
 runs the 512-matrix batched workload instead (FP32 storage, K = 1, 2, 4 or 8 right-hand sides),
 one graph replay per step, at the given schedule or the batch's default; with --one-matrix, a
-batch of the --workload matrix alone (its multi-right-hand-side SpMV).
+batch of the --workload matrix alone (its multi-right-hand-side SpMV); with --one-kernel, the tile
+kernel over the whole batch where it would take work lists.
 """
 from __future__ import annotations
 
@@ -39,6 +40,8 @@ def main() -> None:
                     help="the 512-matrix batched workload at this many right-hand sides")
     ap.add_argument("--one-matrix", action="store_true",
                     help="with --batched: a batch of the --workload matrix alone")
+    ap.add_argument("--one-kernel", action="store_true",
+                    help="with --batched: the tile kernel over the whole batch, no work lists")
     args = ap.parse_args()
     if args.batched:
         run_batched(args)
@@ -70,7 +73,9 @@ def main() -> None:
     assert h.check() == 0, h.last_error
     ms = [p.elapsed_time(q) for p, q in evs]
     src, conf = h.schedule_source()
-    print(f"{args.workload} {args.form} m={a.m} nnz={a.nnz} schedule={h.get_config()} "
+    lanes, slots = h.kernel()
+    kernel = f"row kernel ({lanes} x {slots})" if lanes else f"schedule={h.get_config()}"
+    print(f"{args.workload} {args.form} m={a.m} nnz={a.nnz} {kernel} "
           f"(source {src}, confidence {conf:.3f}): median {statistics.median(ms):.4f} ms "
           f"over {args.steps} steps")
     h.close()
@@ -84,6 +89,8 @@ def run_batched(args) -> None:
     mats = [gen.WORKLOADS[args.workload]()] if args.one_matrix else gen.batch_workload(512)
     cfg = args.config[:3] if args.config else (0, 0, 0)
     b = batch.Batch(mats, k=k, seg=cfg[0], tiles_per_worker=cfg[1], warps_per_cta=cfg[2])
+    if args.one_kernel:
+        b.set_variant(l2_only=b.info()["x_l2_only"])
     x = torch.from_numpy(gen.uniform(b.n * k, 3).reshape(b.n, k).astype(np.float32)).cuda()
     y = torch.zeros((b.m, k), dtype=torch.float32, device="cuda")
     flush = torch.empty(64 << 20, dtype=torch.int32, device="cuda")
@@ -102,8 +109,11 @@ def run_batched(args) -> None:
     ms = statistics.median(p.elapsed_time(q) for p, q in evs)
     info = b.info()
     sched = tuple(args.config[:3]) if args.config else "default"
-    print(f"batched k={k} matrices={len(mats)} nnz={b.nnz} schedule={sched} "
-          f"variant=(one_head {info['one_head']}, l2_only {info['x_l2_only']}): median "
+    kernels = (f"{info['row_lists']} row lists, {info['tile_workers']} tile workers (one_head "
+               f"{info['workers_one_head']}, l2_only {info['workers_x_l2_only']})"
+               if info["row_lists"] else
+               f"variant=(one_head {info['one_head']}, l2_only {info['x_l2_only']})")
+    print(f"batched k={k} matrices={len(mats)} nnz={b.nnz} schedule={sched} {kernels}: median "
           f"{ms:.4f} ms over {args.steps} steps, {b.nnz * k / ms / 1e6:.1f} G nnz*k/s")
     b.close()
 

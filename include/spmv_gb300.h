@@ -99,11 +99,13 @@ int bhsp_set_config(bhsp_spmv* h, int seg, int tiles_per_worker, int warps_per_c
 int bhsp_set_tuner(bhsp_spmv* h, const char* path);
 /* How prepare_mem chose the schedule in use: *source = one of BHSP_SCHEDULE_*, *confidence =
  * the network's probability of its pick (0 when no network ran).  With the environment
- * variable BHSP_LOG_SCHEDULE set (not "0"), prepare_mem also prints the schedule and its
- * source to stderr, so a caller that cannot be changed shows what it got. */
+ * variable BHSP_LOG_SCHEDULE set (not "0"), prepare_mem also prints the schedule, its source and
+ * whether the matrix takes the row kernel, which uses none, to stderr, so a caller that cannot be changed shows what it got. */
 int bhsp_get_schedule_source(const bhsp_spmv* h, int* source, float* confidence);
 int bhsp_get_config(const bhsp_spmv* h, int* seg, int* tiles_per_worker, int* warps_per_cta,
                     int* stages);
+/* The kernel that the prepared handle runs, as bhsp_plan_kernel reports it for a plan. */
+int bhsp_get_kernel(const bhsp_spmv* h, int* lanes, int* slots);
 /* Replace x (host pointer, same type as in prepare_mem) without rebuilding anything; returns
  * once x has been read, so the caller may reuse its buffer.  As prepare_mem does, it reads
  * pageable host memory with a copy kernel where the device accesses pageable memory through the
@@ -160,6 +162,10 @@ int bhsp_plan_check(bhsp_plan* p, void* stream);
 /* Number of device kernels one bhsp_plan_execute launches: 2, or 1 where the plan runs the row
  * kernel (short, even rows: lanes on whole rows) or has no non-zeros. */
 int bhsp_plan_launches(const bhsp_plan* p);
+/* The kernel the next bhsp_plan_execute runs: *lanes = 0 for the tile kernel, which takes the plan's
+ * schedule; else the row kernel, which has none, with *lanes lanes to a row and *slots non-zeros to a
+ * lane. */
+int bhsp_plan_kernel(const bhsp_plan* p, int* lanes, int* slots);
 /* tile_ptr of the plan (device pointer, ntiles+1 entries) and its tile size. */
 int bhsp_plan_tiles(const bhsp_plan* p, const uint32_t** d_tile_ptr, int* ntiles, int* tile_nnz);
 /* The chunk form the plan's tile kernel takes, fixed when the plan is built: *short_rows =
@@ -229,11 +235,16 @@ int bhsp_batch_check(bhsp_batch* b, void* stream);
 /* Tiles and workers of the partition over the whole batch, the grid of the tile workers' kernel
  * and the device kernels of one execute. */
 int bhsp_batch_info(const bhsp_batch* b, int* ntiles, int* nworkers, int* grid, int* launches);
-/* The kernel variant bhsp_batch_create chose for the batch, as bhsp_plan_chunk_form /
+/* The kernel variant bhsp_batch_create chose for the tile kernel over the whole batch, as bhsp_plan_chunk_form /
  * bhsp_plan_gather_path do for one matrix: *one_head = 1 for the branch-free one-head chunk form
  * (one right-hand side and few rows shorter than a chunk), *l2_only = 1 when x is gathered from
  * L2 only (fewer than half of about 2^20 sampled columns lie near their neighbours). */
 int bhsp_batch_variant(const bhsp_batch* b, int* one_head, int* l2_only);
+/* What the next bhsp_batch_execute runs instead where the batch takes work lists: *row_lists row
+ * kernels over lists of row blocks (0: the one tile kernel over all rows, with the variant above),
+ * *tile_workers tile workers for the rows between them, and these workers' variant. */
+int bhsp_batch_lists(const bhsp_batch* b, int* row_lists, int* tile_workers, int* one_head,
+                     int* l2_only);
 /* Overrides that choice: one_head / l2_only = 1 or 0 to force, -1 to keep.  The one-head form
  * exists for one right-hand side only (one_head = 1 with k > 1 is rejected).  Every variant
  * gives the same y; the next bhsp_batch_execute with use_graph captures the graph again.  A batch

@@ -1,0 +1,65 @@
+"""Which kernel a plan, a handle and a batch run, and that a schedule which is set, tuned or reported is
+one of the kernel that it says."""
+import numpy as np
+import pytest
+
+import benchmark_spmv_using_csr_gb300 as sp
+from benchmark_spmv_using_csr_gb300 import batch, gen
+
+pytestmark = pytest.mark.gpu
+
+
+def _plan(vt, a, *cfg):
+    import torch
+    return sp.Plan(vt, a.m, a.n, torch.from_numpy(a.row_ptr).cuda(), torch.from_numpy(a.col).cuda(),
+                   None, *cfg)
+
+
+def _handle(vt, a, cfg=None):
+    h = sp.BhsparseSpmvCuda(vt)
+    if cfg is not None:
+        assert h.set_config(*cfg) == 0, h.last_error
+    dt = sp.host_dtype(vt)
+    y = np.zeros(a.m, dt)
+    assert h.prepare_mem(a.m, a.n, a.nnz, a.row_ptr, a.col, a.val.astype(dt), np.ones(a.n, dt), y) == 0
+    return h, y
+
+
+@pytest.mark.parametrize("vt", [sp.VALUE_F64, sp.VALUE_F32, sp.VALUE_MIXED_F32, sp.VALUE_MIXED_BF16])
+def test_plan_and_handle_report_their_kernel(cuda_ok, capfd, monkeypatch, vt):
+    monkeypatch.setenv("BHSP_LOG_SCHEDULE", "1")
+    for a, kernel in ((gen.stencil3d(30, 30, 30), (1, 28)), (gen.stencil2d(90, 80), (1, 8)),
+                      (gen.powerlaw(20_000, seed=3), (0, 0))):
+        p = _plan(vt, a)
+        assert p.kernel() == kernel and p.launches == (1 if kernel[0] else 2)
+        if kernel[0]:
+            p.set_grid(False)
+            assert p.kernel() == (0, 0)
+            p.set_grid(None)
+            assert p.kernel() == kernel
+            p.set_variant(l2_only=p.gather_path()[2])
+            assert p.kernel() == (0, 0)
+        p.close()
+        capfd.readouterr()
+        h, _ = _handle(vt, a)
+        assert h.kernel() == kernel
+        assert ("row kernel" in capfd.readouterr().err) == (kernel[0] > 0)
+        h.close()
+
+
+@pytest.mark.parametrize("k", [1, 2, 4, 8])
+def test_batch_reports_its_lists(cuda_ok, k):
+    regular, power = gen.stencil3d(40, 40, 40), gen.powerlaw(20_000, seed=3)
+    wide = gen.blockdiag(4096, 4096, 512)
+    for mats, lists, tiles, variant in (([regular] * 2, True, False, (False, False)),
+                                        ([regular, power], True, True, (False, True)),
+                                        ([regular, wide], True, True, (k == 1, False)),
+                                        ([power], False, False, (False, False))):
+        b = batch.Batch(mats, k=k)
+        info = b.info()
+        assert (info["row_lists"] > 0) == lists and (info["tile_workers"] > 0) == tiles
+        assert (info["workers_one_head"], info["workers_x_l2_only"]) == variant
+        b.set_variant(l2_only=info["x_l2_only"])
+        info = b.info()
+        assert info["row_lists"] == info["tile_workers"] == 0 and info["launches"] == 2
+        b.close()
