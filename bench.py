@@ -413,10 +413,12 @@ def run_ours(args) -> None:
     barrier()
     e2e_call_value = whole_job_gbs(world, B, args.steps, e2e_call_s)
     # the same per-call sequence on pageable host arrays, as the reference's driver allocates them
-    # (malloc); a second handle at the same schedule
+    # (malloc); a second handle with the same kernel and schedule
     x_pg, y_pg = x.copy(), np.zeros(a.m)
     h2 = sp.BhsparseSpmvCuda(sp.VALUE_F64)
-    assert h2.set_config(seg, tpw, warps, stages) == 0 and h2.set_device(local) == 0
+    if h.kernel() == (0, 0):
+        assert h2.set_config(seg, tpw, warps, stages) == 0, h2.last_error
+    assert h2.set_device(local) == 0, h2.last_error
     assert h2.prepare_mem(a.m, a.n, a.nnz, a.row_ptr, a.col, a.val, x_pg, y_pg) == 0, h2.last_error
     for _ in range(3):
         assert h2.set_x(x_pg) == 0 and h2.run_benchmark() == 0 and h2.get_y() == 0

@@ -94,7 +94,7 @@ struct bhsp_plan {
     int x_sampled = 0, x_near = 0;  // sampled non-zeros, those with a near column
     bool x_l2 = false;              // the tile kernels gather x from L2 only
     RowForm rows{};                 // lanes > 0: the row kernel runs, unless ...
-    bool variant_set = false;       // ... the caller forced a tile-kernel variant or grid
+    bool variant_set = false;       // ... the caller set a tile-kernel variant, grid or schedule
     int device = 0;
     std::string last_error;
 };
@@ -722,6 +722,7 @@ extern "C" int bhsp_prepare_mem(bhsp_spmv* h, int m, int n, int nnz, const int* 
         return rc;
     }
     h->plan = p;
+    if (h->cfg_user) p->variant_set = true;  // a schedule that the caller set is the one that runs
     if (const char* lg = std::getenv("BHSP_LOG_SCHEDULE"); lg && *lg && *lg != '0') {
         static const char* const kSource[] = {"the caller (bhsp_set_config)", "the fixed default",
                                               "the learned network", "the autotune sweep"};

@@ -88,10 +88,12 @@ int bhsp_set_device(bhsp_spmv* h, int device);
  * 2D tensor copies; a matrix with no full tile runs the direct-load kernel).  Before
  * prepare_mem; 0 for seg / tiles_per_worker / warps_per_cta and -1 for stages take the fixed
  * default (16, 8, 4, 0; stages 2 for BHSP_VALUE_MIXED_BF16, whose staged schedule is the faster
- * one).  Rejected if the staged ring does not fit in shared memory.  Without this call
- * prepare_mem chooses the schedule itself (bhsp_choose_schedule with the handle's network,
- * see bhsp_set_tuner), which is what the reference's callers get: its geometry is a compile-
- * time constant (spmv_cuda/common.h:39-48, spmv_cuda/bhsparse_spmv_cuda.h:323-328). */
+ * one).  Rejected if the staged ring does not fit in shared memory.  A matrix prepared after this
+ * call runs the tile kernel at this schedule, whatever its rows.  Without it prepare_mem chooses
+ * the schedule itself (bhsp_choose_schedule with the handle's network, see bhsp_set_tuner), and a
+ * matrix of short, even rows runs the row kernel, which has none (bhsp_get_kernel).  That is what
+ * the reference's callers get: its geometry is a compile-time constant (spmv_cuda/common.h:39-48,
+ * spmv_cuda/bhsparse_spmv_cuda.h:323-328). */
 int bhsp_set_config(bhsp_spmv* h, int seg, int tiles_per_worker, int warps_per_cta, int stages);
 /* The network prepare_mem consults when bhsp_set_config was not called: NULL = the library's
  * network for the handle's value type (the default; see bhsp_choose_schedule), "" = none (the
@@ -100,7 +102,8 @@ int bhsp_set_tuner(bhsp_spmv* h, const char* path);
 /* How prepare_mem chose the schedule in use: *source = one of BHSP_SCHEDULE_*, *confidence =
  * the network's probability of its pick (0 when no network ran).  With the environment
  * variable BHSP_LOG_SCHEDULE set (not "0"), prepare_mem also prints the schedule, its source and
- * whether the matrix takes the row kernel, which uses none, to stderr, so a caller that cannot be changed shows what it got. */
+ * whether the matrix takes the row kernel, which uses none, to stderr, so a caller that cannot be
+ * changed shows what it got. */
 int bhsp_get_schedule_source(const bhsp_spmv* h, int* source, float* confidence);
 int bhsp_get_config(const bhsp_spmv* h, int* seg, int* tiles_per_worker, int* warps_per_cta,
                     int* stages);
@@ -144,7 +147,9 @@ typedef struct bhsp_plan bhsp_plan;
 
 /* Validates the CSR on the device, builds tile_ptr and allocates the carry records.
  * row_ptr / col_idx stay owned by the caller and must outlive the plan; col_idx must be
- * 32-byte aligned.  The schedule fields are as in bhsp_set_config. */
+ * 32-byte aligned.  The schedule fields are as in bhsp_set_config and are the tile kernel's: a
+ * matrix of short, even rows runs the row kernel, which has no schedule, unless bhsp_plan_set_grid or
+ * bhsp_plan_set_variant asks for the tile kernel (bhsp_plan_kernel reports which). */
 int bhsp_plan_create(bhsp_plan** out, int value_type, int m, int n, int nnz,
                      const int* d_row_ptr, const int* d_col_idx, int seg, int tiles_per_worker,
                      int warps_per_cta, int stages, void* stream);
@@ -180,7 +185,8 @@ int bhsp_plan_gather_path(const bhsp_plan* p, int* sampled, int* near, int* l2_o
 /* Overrides the kernel variant the plan's rules chose: one_head (the chunk form above) and
  * l2_only (the gather path) = 1 or 0 to force it, -1 to keep the rule's choice.  Every variant
  * gives the same y; only the speed differs.  Takes effect at the next bhsp_plan_execute.  A plan
- * with a forced variant or grid runs the tile kernel, whatever its rows. */
+ * with a forced variant or grid runs the tile kernel, whatever its rows; bhsp_plan_set_grid(p, -1)
+ * gives the grid back to the rule, and only a new plan has no forced variant. */
 int bhsp_plan_set_variant(bhsp_plan* p, int one_head, int l2_only);
 /* Overrides the grid of the direct-load tile kernel: 1 = the persistent kernel (warps draw
  * workers from the plan's work queue), 0 = a static grid of one warp per worker, -1 = the rule
@@ -248,7 +254,8 @@ int bhsp_batch_lists(const bhsp_batch* b, int* row_lists, int* tile_workers, int
 /* Overrides that choice: one_head / l2_only = 1 or 0 to force, -1 to keep.  The one-head form
  * exists for one right-hand side only (one_head = 1 with k > 1 is rejected).  Every variant
  * gives the same y; the next bhsp_batch_execute with use_graph captures the graph again.  A batch
- * with a forced variant runs the tile kernel over all its rows. */
+ * with a forced variant, also that which bhsp_batch_variant reports, runs the tile kernel over all its
+ * rows; only a new batch has its work lists again. */
 int bhsp_batch_set_variant(bhsp_batch* b, int one_head, int l2_only);
 /* The batched form's schedule tuner.  Candidates: S 8 / 16 / 32 x 1 / 2 / 4 / 8 tiles per
  * worker x 4 / 8 warps per CTA.  bhsp_batch_autotune builds the batch at every candidate and

@@ -63,3 +63,19 @@ def test_batch_reports_its_lists(cuda_ok, k):
         info = b.info()
         assert info["row_lists"] == info["tile_workers"] == 0 and info["launches"] == 2
         b.close()
+
+
+@pytest.mark.parametrize("vt", [sp.VALUE_F64, sp.VALUE_F32, sp.VALUE_MIXED_F32, sp.VALUE_MIXED_BF16])
+@pytest.mark.parametrize("cfg", [(8, 4, 4, 0), (16, 2, 4, 2), (0, 0, 0, -1)])
+def test_a_schedule_that_the_caller_sets_runs(cuda_ok, vt, cfg):
+    """bhsp_set_config: the handle runs the tile kernel, also on a matrix that takes the row kernel
+    without it, and y is the exact sum."""
+    a = gen.stencil3d(30, 20, 25)
+    a.val = gen.uniform_int(a.nnz, 8, 10) - 4.0
+    want = np.bincount(np.repeat(np.arange(a.m), np.diff(a.row_ptr)), a.val, a.m)
+    for c, rows in ((None, True), (cfg, False)):
+        h, y = _handle(vt, a, c)
+        assert (h.kernel()[0] > 0) == rows
+        assert h.run_benchmark() == 0 and h.get_y() == 0
+        assert (y == want).all()
+        h.close()
