@@ -385,6 +385,8 @@ extern "C" int bhsp_plan_check(bhsp_plan* p, void* stream) {
     return plan_check(p, static_cast<cudaStream_t>(stream));
 }
 
+void spmv::plan_force_tiles(bhsp_plan* p) { p->variant_set = true; }
+
 extern "C" int bhsp_plan_launches(const bhsp_plan* p) {
     if (!p) return 0;
     return p->m == 0 ? 0 : (p->nworkers > 0 && !plan_takes_rows(p) ? 2 : 1);
@@ -722,7 +724,7 @@ extern "C" int bhsp_prepare_mem(bhsp_spmv* h, int m, int n, int nnz, const int* 
         return rc;
     }
     h->plan = p;
-    if (h->cfg_user) p->variant_set = true;  // a schedule that the caller set is the one that runs
+    if (h->cfg_user) spmv::plan_force_tiles(p);  // a schedule that the caller set is the one that runs
     if (const char* lg = std::getenv("BHSP_LOG_SCHEDULE"); lg && *lg && *lg != '0') {
         static const char* const kSource[] = {"the caller (bhsp_set_config)", "the fixed default",
                                               "the learned network", "the autotune sweep"};

@@ -226,6 +226,8 @@ namespace spmv {
 int plan_create_impl(bhsp_plan** out, int value_type, int m, int n, int nnz, const int* d_row_ptr,
                      const int* d_col_idx, int seg, int tiles_per_worker, int warps_per_cta,
                      int stages, void* stream, bool validate);
+// The plan runs the tile kernel at its schedule, whatever its rows.
+void plan_force_tiles(bhsp_plan* p);
 
 // Dynamic shared memory one CTA of the TMA-staged kernel needs (0 for the direct kernel);
 // value_type as in bhsp_value_type.  Configurations above 227 KB cannot run.

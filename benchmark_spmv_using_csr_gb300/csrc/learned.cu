@@ -259,9 +259,26 @@ extern "C" int bhsp_choose_schedule(int value_type, int m, int n, int nnz, const
         if (source) *source = BHSP_SCHEDULE_LEARNED;
         return BHSPARSE_SUCCESS;
     }
-    // a likely slow pick: the full sweep decides (it needs the matrix values and x / y)
+    // a likely slow pick: the full sweep decides (it needs the matrix values and x / y), unless a plan
+    // on this matrix takes the row kernel and the sweep would time what does not run
     if (nnz > 0 && (!d_col_idx || !d_val || !d_x)) return BHSPARSE_INVALID_ARGUMENT;
     if (m > 0 && !d_y) return BHSPARSE_INVALID_ARGUMENT;
+    bhsp_plan* plan = nullptr;
+    rc = spmv::plan_create_impl(&plan, value_type, m, n, nnz, d_row_ptr, d_col_idx, 0, 0, 0, -1,
+                                stream, true);
+    if (rc) return rc;
+    int lanes = 0;
+    bhsp_plan_kernel(plan, &lanes, nullptr);
+    bhsp_plan_destroy(plan);
+    if (lanes > 0) {
+        if (!runnable) return fixed_default(value_type, seg, tiles_per_worker, warps_per_cta, stages);
+        *seg = c[0];
+        *tiles_per_worker = c[1];
+        *warps_per_cta = c[2];
+        *stages = c[3];
+        if (source) *source = BHSP_SCHEDULE_LEARNED;
+        return BHSPARSE_SUCCESS;
+    }
     const int K = bhsp_tune_num_candidates();
     std::vector<float> ms((size_t)K, 0.f);
     int best = -1;

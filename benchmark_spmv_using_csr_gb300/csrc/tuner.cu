@@ -2,7 +2,9 @@
 //
 // The autotuner times every candidate schedule (non-zeros per lane S, tiles per worker,
 // warps per CTA, direct or TMA-staged stream) of the tile kernel on the caller's matrix and reports the per-candidate time
-// and the fastest.  It only picks a schedule; every candidate computes the same y (the
+// and the fastest, also for a matrix whose plan takes the row kernel: its table is of the tile kernel,
+// and a cache keyed by the row lengths may serve it to a matrix with other columns, which runs that
+// kernel.  It only picks a schedule; every candidate computes the same y (the
 // arithmetic does not depend on the schedule beyond summation order).  No counterpart in the
 // reference, whose tile geometry is fixed at compile time (spmv_cuda/common.h:39-48).
 #include <algorithm>
@@ -85,6 +87,7 @@ extern "C" int bhsp_autotune(int value_type, int m, int n, int nnz, const int* d
         rc = spmv::plan_create_impl(&p, value_type, m, n, nnz, d_row_ptr, d_col_idx, c.seg,
                                     c.tiles_per_worker, c.warps_per_cta, c.stages, stream, false);
         if (rc) break;
+        spmv::plan_force_tiles(p);  // a row kernel has no schedule to time
         for (int w = 0; w < warmup && rc == 0; ++w) rc = bhsp_plan_execute(p, d_val, d_x, d_y, stream);
         for (int r = 0; r < reps && rc == 0; ++r) {
             if (flush && cudaMemsetAsync(flush, r & 0xff, flush_bytes, st) != cudaSuccess)

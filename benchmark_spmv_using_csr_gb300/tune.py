@@ -42,7 +42,8 @@ def _stream_ptr(stream) -> int:
 
 def autotune(value_type: int, row_ptr, col_idx, val, x, y, n: int | None = None,
              warmup: int = 2, reps: int = 5, stream=None) -> tuple[np.ndarray, int]:
-    """Time every candidate schedule on torch CUDA tensors; returns (ms per candidate, best)."""
+    """Time every candidate schedule of the tile kernel on torch CUDA tensors (also where a plan on
+    the matrix would run the row kernel); returns (ms per candidate, best)."""
     L = lib()
     k = L.bhsp_tune_num_candidates()
     ms = np.zeros(k, np.float32)

@@ -283,12 +283,12 @@ void bhsp_batch_destroy(bhsp_batch* b);
 int bhsp_tune_num_candidates(void);
 int bhsp_tune_candidate(int index, int* seg, int* tiles_per_worker, int* warps_per_cta,
                         int* stages);
-/* Autotuner: validates the CSR, then times y = A.x for every candidate on the given device
- * buffers (`warmup` untimed runs, then the median of `reps` CUDA-event-timed runs, each
- * preceded by a write of twice the L2 size so that it starts with the matrix and x out of L2)
- * and writes ms_out[bhsp_tune_num_candidates()] and the index of the fastest to *best.  A
- * staged candidate whose ring does not fit in shared memory for this value type is not run and
- * gets +infinity.  Synchronous. */
+/* Autotuner: validates the CSR, then times y = A.x by the tile kernel for every candidate on the
+ * given device buffers (`warmup` untimed runs, then the median of `reps` CUDA-event-timed runs,
+ * each preceded by a write of twice the L2 size so that it starts with the matrix and x out of L2),
+ * also for a matrix whose plan runs the row kernel, and writes ms_out[bhsp_tune_num_candidates()]
+ * and the index of the fastest to *best.  A staged candidate whose ring does not fit in shared
+ * memory for this value type is not run and gets +infinity.  Synchronous. */
 int bhsp_autotune(int value_type, int m, int n, int nnz, const int* d_row_ptr,
                   const int* d_col_idx, const void* d_val, const void* d_x, void* d_y, int warmup,
                   int reps, float* ms_out, int* best, void* stream);
@@ -303,8 +303,9 @@ int bhsp_autotune(int value_type, int m, int n, int nnz, const int* d_row_ptr,
  * probabilities and entropy in, the probability that the pick is below 95 % of the best time
  * out) rates the pick as likely slow, or the pick's probability is below the file's confidence
  * threshold; then the full autotune sweep (bhsp_autotune, 1 warm-up and the median of 3
- * flushed-L2 runs per candidate, writing d_y) decides.  *confidence is the first network's
- * probability of its pick.  tuner_path: NULL = the library's network for value_type, the file
+ * flushed-L2 runs per candidate, writing d_y) decides.  A matrix whose plan runs the row
+ * kernel has no sweep: the network's pick stays, for a caller who forces the tile kernel.
+ * *confidence is the first network's probability of its pick.  tuner_path: NULL = the library's network for value_type, the file
  * tuner_data/gb300_<f64|f32|mixed_f32|mixed_bf16>_tuner.bin next to the library (or in the
  * directory named by the BHSP_TUNER_DIR environment variable); with no such file the fixed
  * default is returned (*source = BHSP_SCHEDULE_DEFAULT).  "" = no network (the fixed default).
