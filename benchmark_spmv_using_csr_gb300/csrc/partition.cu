@@ -128,9 +128,14 @@ cudaError_t launch_bitflags(const int* row_ptr, int m, int nnz, int seg, const u
 //    chunk of cw slots (heads at s and s + len share an aligned chunk only if len < cw), and it
 //    does so in at most one chunk.
 //  * What the row kernel needs: see RowCounts.
+// The warps' counts meet in shared memory first: an atomic per warp and count on the few global
+// addresses took 56 us on 4.2 M rows, an atomic per CTA 19 us.
 __global__ void k_row_counts(const int* __restrict__ row_ptr, int m, int cw,
                              RowCounts* __restrict__ counts) {
     const long long stride = (long long)gridDim.x * blockDim.x;  // 64-bit: m may be near 2^31
+    __shared__ RowCounts s;
+    if (threadIdx.x == 0) s = RowCounts{};
+    __syncthreads();
     const int lane = threadIdx.x & 31;
     unsigned shorts = 0, top = 0, eights = 0;
     unsigned long long groups[4] = {0, 0, 0, 0};
@@ -157,12 +162,19 @@ __global__ void k_row_counts(const int* __restrict__ row_ptr, int m, int cw,
         for (int t = 0; t < 4; ++t) groups[t] += __shfl_xor_sync(SPMV_FULL_MASK, groups[t], d);
     }
     if (lane == 0) {
-        if (shorts) atomicAdd(&counts->short_rows, (unsigned long long)shorts);
-        if (eights) atomicAdd(&counts->eights, (unsigned long long)eights);
-        if (top) atomicMax(&counts->max_len, (unsigned long long)top);
+        atomicAdd(&s.short_rows, (unsigned long long)shorts);
+        atomicAdd(&s.eights, (unsigned long long)eights);
+        atomicMax(&s.max_len, (unsigned long long)top);
 #pragma unroll
-        for (int t = 0; t < 4; ++t)
-            if (groups[t]) atomicAdd(&counts->groups[t], groups[t]);
+        for (int t = 0; t < 4; ++t) atomicAdd(&s.groups[t], groups[t]);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicAdd(&counts->short_rows, s.short_rows);
+        atomicAdd(&counts->eights, s.eights);
+        atomicMax(&counts->max_len, s.max_len);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) atomicAdd(&counts->groups[t], s.groups[t]);
     }
 }
 
