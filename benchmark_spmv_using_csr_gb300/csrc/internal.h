@@ -198,13 +198,13 @@ struct BatchWork {
     bool one_head = false, x_l2 = false;
 };
 // What the work lists need of each block of 256 rows.
-struct BlockStat {
-    int first;      // its first non-zero
-    int max_len;    // the longest row
-    int groups[4];  // as RowCounts::groups, over this block
-    int eights;     // non-empty rows of a multiple of 8 non-zeros
-    int filled;     // non-empty rows
-    int shorts;     // non-empty rows shorter than cw non-zeros
+struct BlockStat {  // (small: creating a batch copies one per block to the host)
+    int first;               // its first non-zero
+    uint16_t max_len;        // the longest row, at most 0xffff
+    uint16_t groups[4];      // as RowCounts::groups, over this block, at most 0xffff
+    uint16_t eights;         // non-empty rows of a multiple of 8 non-zeros
+    uint16_t filled;         // non-empty rows
+    uint16_t shorts;         // non-empty rows shorter than cw non-zeros
     uint32_t sampled, near;  // of its every step-th non-zeros, as launch_x_locality counts them
 };
 cudaError_t launch_block_stats(const int* row_ptr, const int* col, int m, int nnz, int cw, int step,

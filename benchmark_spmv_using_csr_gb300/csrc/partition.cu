@@ -247,27 +247,35 @@ __global__ void k_block_stats(const int* __restrict__ row_ptr, int m, int nblock
     const int lane = threadIdx.x & 31;
     const int nwarps = gridDim.x * (blockDim.x >> 5);
     for (int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); b < nblocks; b += nwarps) {
-        BlockStat s{};
-        s.first = __ldg(row_ptr + b * BATCH_BLOCK);
+        int max_len = 0, eights = 0, filled = 0, shorts = 0, groups[4] = {0, 0, 0, 0};
         for (int i = 0; i < BATCH_BLOCK; i += 32) {
             const long long r = (long long)b * BATCH_BLOCK + i + lane;
             const int lo = r < m ? __ldg(row_ptr + r) : 0;
             const int len = r < m ? __ldg(row_ptr + r + 1) - lo : 0;
-            s.filled += __popc(__ballot_sync(SPMV_FULL_MASK, len > 0));
-            s.eights += __popc(__ballot_sync(SPMV_FULL_MASK, len > 0 && len % 8 == 0));
-            s.shorts += __popc(__ballot_sync(SPMV_FULL_MASK, len > 0 && len < cw));
+            filled += __popc(__ballot_sync(SPMV_FULL_MASK, len > 0));
+            eights += __popc(__ballot_sync(SPMV_FULL_MASK, len > 0 && len % 8 == 0));
+            shorts += __popc(__ballot_sync(SPMV_FULL_MASK, len > 0 && len < cw));
             int most = len;
 #pragma unroll
             for (int t = 3, d = 1; t >= 0; --t) {
                 const int rows = 32 >> t;
                 for (; d < rows; d <<= 1) most = max(most, __shfl_xor_sync(SPMV_FULL_MASK, most, d));
-                s.groups[t] += (lane & (rows - 1)) == 0 ? (int)((most + (4LL << t) - 1) >> (2 + t)) : 0;
+                groups[t] += (lane & (rows - 1)) == 0 ? min((int)((most + (4LL << t) - 1) >> (2 + t)), 0x7fff) : 0;
             }
-            s.max_len = max(s.max_len, most);
+            max_len = max(max_len, most);
         }
 #pragma unroll
-        for (int t = 0; t < 4; ++t) s.groups[t] = __reduce_add_sync(SPMV_FULL_MASK, s.groups[t]);
-        if (lane == 0) stat[b] = s;
+        for (int t = 0; t < 4; ++t) groups[t] = __reduce_add_sync(SPMV_FULL_MASK, groups[t]);
+        if (lane == 0) {
+            BlockStat s{};
+            s.first = __ldg(row_ptr + b * BATCH_BLOCK);
+            s.max_len = (uint16_t)min(max_len, 0xffff);
+            for (int t = 0; t < 4; ++t) s.groups[t] = (uint16_t)min(groups[t], 0xffff);
+            s.eights = (uint16_t)eights;
+            s.filled = (uint16_t)filled;
+            s.shorts = (uint16_t)shorts;
+            stat[b] = s;
+        }
     }
 }
 
@@ -275,12 +283,20 @@ __global__ void k_block_stats(const int* __restrict__ row_ptr, int m, int nblock
 __global__ void k_block_locality(const int* __restrict__ row_ptr, const int* __restrict__ col,
                                  int m, int nnz, int step, BlockStat* __restrict__ stat) {
     const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s * step < nnz;
-         s += stride) {
+    const int lane = threadIdx.x & 31;
+    for (long long s0 = blockIdx.x * (long long)blockDim.x + threadIdx.x - lane; s0 * step < nnz;
+         s0 += stride) {  // warp-uniform
+        const long long j = (s0 + lane) * step;
         int row = 0;
-        const bool near = near_column(row_ptr, col, m, (int)(s * step), &row);
-        atomicAdd(&stat[row / BATCH_BLOCK].sampled, 1u);
-        if (near) atomicAdd(&stat[row / BATCH_BLOCK].near, 1u);
+        const bool near = j < nnz && near_column(row_ptr, col, m, (int)j, &row);
+        // one pair of atomics for the lanes of a block, which are neighbours
+        const unsigned lanes =
+            __match_any_sync(SPMV_FULL_MASK, j < nnz ? row / BATCH_BLOCK : -1);
+        const unsigned hits = __ballot_sync(SPMV_FULL_MASK, near) & lanes;
+        if (j < nnz && lane == __ffs(lanes) - 1) {
+            atomicAdd(&stat[row / BATCH_BLOCK].sampled, (uint32_t)__popc(lanes));
+            if (hits) atomicAdd(&stat[row / BATCH_BLOCK].near, (uint32_t)__popc(hits));
+        }
     }
 }
 
