@@ -17,8 +17,8 @@
 // Measured on the 27-point stencil on 160^3 (109 M non-zeros), tile kernel at its best schedule
 // -> this one: mixed FP32 176 -> 136 us (6800 GB/s: memory-bound), FP64 262 -> 229 us (6090 GB/s;
 // the FP64 pipe needs 195 us for its 28 slots a row, memory 208 us); BF16 storage on 121 x 97 x
-// 143 86 -> 49.5 us (5800 GB/s); the 5-point stencil on 256^2, FP64, 8.7 -> 7.2 us (the host's
-// launch path).
+// 143 86 -> 49.5 us (5800 GB/s); the 5-point stencil on 256^2, FP64, 8.6-8.9 -> 6.5-7.4 us (the
+// host's launch path).
 //
 // Random columns: Poisson rows of 8, 8 M non-zeros, mixed FP32 46 -> 38 us (a gather's sector per
 // slot: 227 G/s, the L2-to-SM rate for random sectors being 290-320); read from L2 only they are

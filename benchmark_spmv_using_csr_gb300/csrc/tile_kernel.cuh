@@ -771,9 +771,9 @@ __device__ __forceinline__ R rec_shfl(const R& v, int d) {
 // Bound by the latency of its few dependent loads, which nothing hides: the rows and the records
 // come in one round, and a run behind the warp U records a lane at a time.  One round per
 // dependent load, as it was (rows, neighbours, records, 32 records of a run at a time), cost the
-// dense-row matrix of 1M rows 61.2 us per product in FP64 where it now takes 58.8, the power-law
-// matrix of 700K rows 61.3 -> 57.9 (mixed FP32), and, at 256 non-zeros per worker (4000 records in
-// the longest run), 114 -> 62 us.
+// power-law matrix of 700K rows 60.5 us per product in mixed FP32 where it now takes 56.9, the
+// dense-row matrix of 1M rows 60.5 -> 58.7 (FP64; on other boxes within their noise) and, at 256
+// non-zeros per worker (4000 records in the longest run), 114 -> 62 us.
 // The kernel that calls this begins while the one that writes the records and y still runs, and waits
 // for it (griddepcontrol.wait) first.  So none of the three pointers is declared __restrict__: const
 // __restrict__ data may be read by the non-coherent load, which is defined only for data that nobody
