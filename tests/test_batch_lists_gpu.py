@@ -1,4 +1,5 @@
-"""The batched form over work lists: the kernel variant of its tile workers."""
+"""The batched form over work lists: the kernel variant and the tiles of its tile workers, calls on changing
+buffers, and the tuner on it."""
 import numpy as np
 import pytest
 
@@ -8,7 +9,7 @@ pytestmark = pytest.mark.gpu
 
 
 def _us(b, x, y):
-    """Microseconds per execute: the median of 5 runs of 20."""
+    """Microseconds per execute: the least of 5 runs of 20 after a first one."""
     import torch
     out = []
     for _ in range(6):
@@ -19,7 +20,7 @@ def _us(b, x, y):
         e1.record()
         torch.cuda.synchronize()
         out.append(e0.elapsed_time(e1) * 50)
-    return sorted(out[1:])[2]
+    return min(out[1:])
 
 
 @pytest.mark.parametrize("kind,k", [("wide", 1), ("wide", 2), ("long", 1)])
@@ -131,7 +132,7 @@ def test_changing_buffers_cost_no_capture_per_call(cuda_ok, k):
             e1.record()
             torch.cuda.synchronize()
             out.append(e0.elapsed_time(e1) * 25)
-        return sorted(out[1:])[2]
+        return min(out[1:])
 
     direct = per_call(False, True)
     turns = per_call(True, True)
