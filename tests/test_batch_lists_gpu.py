@@ -46,14 +46,14 @@ def test_long_rows_between_row_blocks_are_no_slower_than_the_one_kernel(cuda_ok,
     assert lists <= 1.1 * one, (lists, one)
 
 
-@pytest.mark.parametrize("rows,k", [(6000, 1), (14_000, 1), (6000, 8)])
-def test_default_tiles_per_worker_of_long_rows(cuda_ok, rows, k):
+@pytest.mark.parametrize("rows,count,k", [(6000, 2, 1), (7000, 4, 1), (6000, 2, 8)])
+def test_default_tiles_per_worker_of_long_rows(cuda_ok, rows, count, k):
     """Rows of 300 to 1500 random columns alone: the default schedule takes at most 1.05 times what 4
     tiles per worker take."""
     import torch
     rng = np.random.default_rng(3)
     a = gen.from_row_lengths(rng.integers(300, 1500, rows), 50_000, seed=9)
-    b = batch.Batch([a] * 2, k=k)
+    b = batch.Batch([a] * count, k=k)
     x = torch.rand(b.n, k, device="cuda")
     y = torch.empty(b.m, k, device="cuda")
     default = _us(b, x, y)
